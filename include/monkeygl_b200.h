@@ -327,6 +327,21 @@ int mk_dvr_backward(const mk_dvr_params *views, int nviews, const float *volume,
                     const float *workspace, const float *grad_images, float *grad_lut,
                     float *grad_volume, void *stream);
 
+/* The two calls above with device scratch memory (256-byte aligned, only
+ * used during the call): the volume is rearranged into bricks in it, which is
+ * several times faster for all but small images of large volumes.  Results
+ * are those of the plain calls (images and workspace bit for bit; gradients
+ * up to the order of their sums).  mk_dvr_scratch_bytes gives the bytes, 0
+ * where the plain calls are as fast; gradients = 1 for a backward call with
+ * grad_volume.  With less (or NULL) scratch they are the plain calls. */
+int mk_dvr_scratch_bytes(const mk_dvr_params *views, int nviews, int gradients, size_t *bytes);
+int mk_dvr_forward_scratch(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
+                           float *images, float *transmittance, float *workspace, void *scratch,
+                           size_t scratch_bytes, void *stream);
+int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
+                            const float *workspace, const float *grad_images, float *grad_lut,
+                            float *grad_volume, void *scratch, size_t scratch_bytes, void *stream);
+
 /*
  * mk_render_cpr without any device allocation.  It has no counterpart in
  * MonkeyGL: it is for callers that cannot call cudaMalloc (a host with a

@@ -160,6 +160,10 @@ _SIGS = {
     "mk_dvr_workspace_floats": (C.c_int, [C.POINTER(DVRParams), C.c_int, C.POINTER(C.c_size_t)]),
     "mk_dvr_forward": (C.c_int, [C.POINTER(DVRParams), C.c_int] + [C.c_void_p] * 6),
     "mk_dvr_backward": (C.c_int, [C.POINTER(DVRParams), C.c_int] + [C.c_void_p] * 7),
+    "mk_dvr_scratch_bytes": (C.c_int, [C.POINTER(DVRParams), C.c_int, C.c_int, C.POINTER(C.c_size_t)]),
+    "mk_dvr_forward_scratch": (C.c_int, [C.POINTER(DVRParams), C.c_int] + [C.c_void_p] * 6 + [C.c_size_t, C.c_void_p]),
+    "mk_dvr_backward_scratch": (C.c_int, [C.POINTER(DVRParams), C.c_int] + [C.c_void_p] * 7 +
+                                [C.c_size_t, C.c_void_p]),
     "mk_server_create": (C.c_int, [C.POINTER(ServerConfig), C.POINTER(C.c_void_p)]),
     "mk_server_destroy": (C.c_int, [C.c_void_p]),
     "mk_server_add_volume": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p,

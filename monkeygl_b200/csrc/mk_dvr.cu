@@ -30,6 +30,7 @@
 // combined by warp shuffles before the shared-memory bins, which go to global
 // memory once per block; the voxel sums take eight global reductions.
 #include <cuda_runtime.h>
+#include <float.h>
 #include <limits.h>
 #include <math.h>
 #include <stdint.h>
@@ -327,6 +328,10 @@ __device__ __forceinline__ void flush_vol(float *__restrict__ gv, const DvrBatch
     }
 }
 
+__device__ __forceinline__ bool gradient_finite(float r, float g, float b) {
+    return fabsf(r) + fabsf(g) + fabsf(b) <= FLT_MAX;
+}
+
 // Reverse march.  A ray walks its samples from the last to the first,
 // reconstructing T_i = T_{i+1} / (1 - a_i) from the transmittance saved after
 // its last sample; at every checkpoint (each 2^ckpt_shift samples) T is taken
@@ -335,8 +340,10 @@ __device__ __forceinline__ void flush_vol(float *__restrict__ gv, const DvrBatch
 // by) takes T_i by re-marching forward from its interval's checkpoint.  Each
 // sample is fetched once otherwise.  The walk is warp-uniform (lanes past
 // their first sample idle), so the LUT-gradient runs that end in one step
-// can be combined across the warp.
-template <bool VOLGRAD>
+// can be combined across the warp.  ODD: only the rays whose
+// pixel gradient is not finite (after k_dvr_backward_bricks, which leaves them
+// out).
+template <bool VOLGRAD, bool ODD>
 __global__ void __launch_bounds__(128) k_dvr_backward(const __grid_constant__ DvrBatch B,
                                                       const float *__restrict__ vol,
                                                       const float4 *__restrict__ lut_g,
@@ -347,25 +354,29 @@ __global__ void __launch_bounds__(128) k_dvr_backward(const __grid_constant__ Dv
     const int n = B.lut_len;
     float4 *L = sm, *D = sm + n;
     float *bins = reinterpret_cast<float *>(sm + 2 * n);
-    load_lut(lut_g, L, D, n);
-    for (int i = threadIdx.x; i < 4 * n; i += blockDim.x) bins[i] = 0.0f;
-    __syncthreads();
-
     const DvrView &V = B.v[blockIdx.z];
     const int x = pixel_x(blockIdx.x, 16), y = pixel_y(blockIdx.y, 16);
     const bool in_image = x < B.W && y < B.H;
     const size_t npix = (size_t)B.W * B.H, pix = in_image ? (size_t)y * B.W + x : 0;
-    const float *wk = work + V.work_off;
     const size_t o = (size_t)blockIdx.z * npix + pix;
     float gr = 0.f, gg = 0.f, gb = 0.f, T = 0.f;
-    int ns = 0;
     if (in_image) {
         gr = grad_images[3 * o];
         gg = grad_images[3 * o + 1];
         gb = grad_images[3 * o + 2];
+    }
+    if (ODD && !__syncthreads_or(!gradient_finite(gr, gg, gb))) return;
+    load_lut(lut_g, L, D, n);
+    for (int i = threadIdx.x; i < 4 * n; i += blockDim.x) bins[i] = 0.0f;
+    __syncthreads();
+
+    const float *wk = work + V.work_off;
+    int ns = 0;
+    if (in_image) {
         ns = reinterpret_cast<const int *>(wk + (size_t)V.max_ckpt * npix)[pix];
         T = wk[(size_t)(V.max_ckpt + 1) * npix + pix];
         if (gr == 0.0f && gg == 0.0f && gb == 0.0f) ns = 0;
+        if (ODD && gradient_finite(gr, gg, gb)) ns = 0;
     }
     const Ray r = make_ray(B, V, x, y);
     const int cmask = (1 << V.ckpt_shift) - 1;
@@ -466,6 +477,596 @@ __global__ void __launch_bounds__(128) k_dvr_backward(const __grid_constant__ Dv
 }
 
 // ---------------------------------------------------------------------------
+// Bricked path (scratch given): the volume is rearranged, per call, into
+// bricks of 8^3 cells before the rays are marched.
+//
+// A ray sample reads the eight voxels of its cell.  In the x-fastest volume
+// the 32 lanes of a warp, whose pixels spread over a plane across the rays,
+// touch up to 24 different 128-byte lines with each of the eight loads, and
+// the kernels above run at the rate at which the load/store unit takes lines
+// (about 190 cycles per warp and sample, 99% of L1TEX).  On 256^3 with eight
+// views of 256^2 the rearrangement takes 66-77 us, the forward 640 us (plain:
+// 5.2 ms) and the backward 1430 us (plain: 6.2 ms); the load/store unit (78%)
+// and instruction issue (73%) now share the bound.  Here a cell's plane
+// of four voxels is one float4 ("quad"), so a sample is two 16-byte loads;
+// a 128-byte line holds 4x2 cells of one plane, and a quarter warp (the lanes
+// a 16-byte load serves together) covers 4x2 pixels.
+//
+// A brick holds the 8x8x9 quads of its cells (its last plane is the next
+// brick's first, kept twice so that a cell never needs two bricks), and is
+// built only if a sample in it can matter, which the LUT decides from the
+// brick's smallest and largest voxel:
+//  * forward: where every LUT entry the brick can reach has alpha 0, a sample
+//    leaves colour and transmittance as they are ("clear" brick);
+//  * backward: there the only gradient is dL/dalpha of those entries.  Where
+//    in addition all voxels of the brick are equal (padding, clipped air),
+//    every sample in it adds the same term, which is added once, times the
+//    number of samples ("flat" brick).
+// Byte maps of the Chebyshev distance to the next brick that is not clear
+// (forward) or not flat (backward) let a ray leave such regions in one step.
+//
+// Cell (ix, iy, iz), ix = -1 .. X-1, has cell coordinates (ix+1, ...); cells
+// at the border repeat the edge voxel, which is the clamping above.
+
+constexpr int kDvrBrickQuads = 576;      // 8 x 8 x 9
+constexpr float kDvrExitMargin = 0.05f;  // cells; covers the rounding of the linear exit model
+
+struct DvrBricks {
+    int nb[3];
+    const float4 *quads;
+    float4 *gquads;                      // voxel gradients in the same layout (backward)
+    const uint8_t *dist;                 // per brick; 0: its samples are evaluated
+    const float *flat;                   // per flat brick: the value of its voxels (backward)
+};
+
+// Offset of a cell's first quad inside its brick (the second is 64 further).
+__device__ __forceinline__ int quad_offset(int lx, int ly, int lz) {
+    return lz * 64 + (ly >> 1) * 16 + (lx >> 2) * 8 + (ly & 1) * 4 + (lx & 3);
+}
+
+// One block per row of four bricks: their 33 x 9 x 9 voxels (a warp reads a
+// row of them, lane = x), each brick's range, the LUT entries it can reach,
+// and, for a needed brick, its quads (and zeroed gradient quads).  The lanes
+// keep the range of their column over the rows, so the ranges cost two
+// instructions a row and one reduction a block.
+template <bool BACKWARD>
+__global__ void __launch_bounds__(256) k_dvr_build(int X, int Y, int Z, int nbx, const float *__restrict__ vol,
+                                                   const float4 *__restrict__ lut, int n, float4 *__restrict__ quads,
+                                                   float4 *__restrict__ gquads, uint8_t *__restrict__ needed,
+                                                   float *__restrict__ flat) {
+    __shared__ float v[81][33];
+    __shared__ float s_lo[8][33], s_hi[8][33];
+    __shared__ int s_need[4];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int x0 = blockIdx.x * 32 - 1, y0 = blockIdx.y * 8 - 1, z0 = blockIdx.z * 8 - 1;
+    const int gx = min(max(x0 + lane, 0), X - 1), gx32 = min(x0 + 32, X - 1);
+    float lo = INFINITY, hi = -INFINITY, lo32 = INFINITY, hi32 = -INFINITY;
+    bool odd = false;                    // a value the range test cannot place
+#pragma unroll
+    for (int t = 0; t < 11; ++t) {
+        const int row = t * 8 + warp, lz = row / 9, ly = row - lz * 9;
+        if (row >= 81) break;
+        const int gy = min(max(y0 + ly, 0), Y - 1), gz = min(max(z0 + lz, 0), Z - 1);
+        const float *p = vol + ((size_t)gz * Y + gy) * X;
+        const float a = __ldg(p + gx);
+        v[row][lane] = a;
+        odd |= !(fabsf(a) <= 2.0f);      // (beyond, the rounding could pass an entry)
+        lo = fminf(lo, a);
+        hi = fmaxf(hi, a);
+        if (lane == 0) {
+            const float e = __ldg(p + gx32);
+            v[row][32] = e;
+            odd |= !(fabsf(e) <= 2.0f);
+            lo32 = fminf(lo32, e);
+            hi32 = fmaxf(hi32, e);
+        }
+    }
+    s_lo[warp][lane] = lo;
+    s_hi[warp][lane] = hi;
+    if (lane == 0) {
+        s_lo[warp][32] = lo32;
+        s_hi[warp][32] = hi32;
+    }
+    odd = __syncthreads_or(odd);
+    if (warp < 4) {
+        // warp j: brick j, columns 8 j .. 8 j + 8
+        lo = INFINITY;
+        hi = -INFINITY;
+        for (int i = lane; i < 72; i += 32) {
+            lo = fminf(lo, s_lo[i / 9][warp * 8 + i % 9]);
+            hi = fmaxf(hi, s_hi[i / 9][warp * 8 + i % 9]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        // entries a sample between lo and hi can reach, one more on each
+        // side for the rounding of the interpolation
+        bool seen = odd;
+        if (!odd) {
+            const float a = fminf(fmaxf(__fmaf_rn(lo, (float)n, -0.5f), 0.0f), (float)(n - 1));
+            const float b = fminf(fmaxf(__fmaf_rn(hi, (float)n, -0.5f), 0.0f), (float)(n - 1));
+            const int i0 = max((int)a - 1, 0), i1 = min((int)b + 2, n - 1);
+            for (int i = i0 + lane; i <= i1; i += 32) {
+                const float4 c = __ldg(lut + i);
+                // a colour that is not finite would show even at alpha 0
+                seen |= c.w != 0.0f || !(fabsf(c.x) <= FLT_MAX && fabsf(c.y) <= FLT_MAX && fabsf(c.z) <= FLT_MAX);
+            }
+        }
+        seen = __any_sync(0xffffffffu, seen);
+        if (lane == 0) {
+            const int bx = blockIdx.x * 4 + warp;
+            const int need = bx >= nbx ? 0 : seen ? 2 : BACKWARD && lo != hi ? 1 : 0;
+            s_need[warp] = need;
+            if (bx < nbx) {
+                const size_t b = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * nbx + bx;
+                needed[b] = (uint8_t)need;
+                if (BACKWARD) flat[b] = lo;
+            }
+        }
+    }
+    __syncthreads();
+    const size_t b0 = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * nbx + blockIdx.x * 4;
+    // 64 threads a brick, one per cell of a plane
+    const int j = tid >> 6, r = tid & 63, need = s_need[j];
+    if (need == 0) return;
+    const int lx = j * 8 + ((r & 3) | ((r >> 1) & 4)), ly = ((r >> 2) & 1) | ((r >> 3) & 6);
+    float4 *q = quads + (b0 + j) * kDvrBrickQuads + r;
+    float4 *g = BACKWARD && gquads && need == 2 ? gquads + (b0 + j) * kDvrBrickQuads + r : nullptr;
+#pragma unroll
+    for (int lz = 0; lz < 9; ++lz) {
+        const float *p = &v[lz * 9 + ly][lx];
+        q[lz * 64] = make_float4(p[0], p[1], p[33], p[34]);
+        // where nothing is seen no voxel has a gradient
+        if (g) g[lz * 64] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+// The gradient quads of one brick, summed per voxel and added to the gradient
+// volume (voxels on a brick's faces get a sum from each brick).
+__global__ void __launch_bounds__(256) k_dvr_fold(int X, int Y, int Z, const float4 *__restrict__ gquads,
+                                                  const uint8_t *__restrict__ needed, float *__restrict__ grad_vol) {
+    __shared__ float4 q[kDvrBrickQuads];
+    const size_t b = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    if (needed[b] != 2) return;
+    for (int i = threadIdx.x; i < kDvrBrickQuads; i += 256) q[i] = gquads[b * kDvrBrickQuads + i];
+    __syncthreads();
+    const int x0 = blockIdx.x * 8 - 1, y0 = blockIdx.y * 8 - 1, z0 = blockIdx.z * 8 - 1;
+    for (int i = threadIdx.x; i < 729; i += 256) {
+        const int lx = i % 9, ly = (i / 9) % 9, lz = i / 81;
+        float s = 0.0f;
+        if (lx < 8 && ly < 8) s += q[quad_offset(lx, ly, lz)].x;
+        if (lx > 0 && ly < 8) s += q[quad_offset(lx - 1, ly, lz)].y;
+        if (lx < 8 && ly > 0) s += q[quad_offset(lx, ly - 1, lz)].z;
+        if (lx > 0 && ly > 0) s += q[quad_offset(lx - 1, ly - 1, lz)].w;
+        if (s == 0.0f) continue;
+        const int gx = min(max(x0 + lx, 0), X - 1), gy = min(max(y0 + ly, 0), Y - 1), gz = min(max(z0 + lz, 0), Z - 1);
+        atomicAdd(grad_vol + ((size_t)gz * Y + gy) * X + gx, s);
+    }
+}
+
+// Cell coordinates and weights of sample i: sample_cell with the cell counted
+// from -1.  The floor is an addition of 1.5 * 2^23 rounded down (exact for
+// the |c| < 2^22 there are; floorf and the conversion to int would go through
+// the quarter-rate unit), and the sample number is kept as a float.  The
+// samples of a ray lie in the cells -1 .. X-1 (to a few hundredths, see
+// use_bricks); inside a known brick only the low three bits are used.
+struct BrickCell {
+    int x, y, z;
+    float wx, wy, wz;
+};
+
+__device__ __forceinline__ void floor_cell(float c, int &i, float &w) {
+    const float magic = 12582912.0f;     // 0x4b400000
+    const float t = __fadd_rd(c, magic);
+    i = __float_as_int(t) - (0x4b400000 - 1);
+    w = c - (t - magic);
+}
+
+__device__ __forceinline__ BrickCell brick_cell(const DvrBatch &B, const Ray &r, float step, float i) {
+    const float a = __fmaf_rn(i, step, r.a0);
+    BrickCell q;
+    floor_cell(__fmaf_rn(__fmaf_rn(a, r.dx, r.px), B.fdim[0], -0.5f), q.x, q.wx);
+    floor_cell(__fmaf_rn(__fmaf_rn(a, r.dy, r.py), B.fdim[1], -0.5f), q.y, q.wy);
+    floor_cell(__fmaf_rn(__fmaf_rn(a, r.dz, r.pz), B.fdim[2], -0.5f), q.z, q.wz);
+    return q;
+}
+
+// The brick of a cell (clamped to those there are).
+__device__ __forceinline__ uint32_t brick_of(const DvrBatch &B, const DvrBricks &K, BrickCell &c) {
+    c.x = min(max(c.x, 0), B.dim[0]);
+    c.y = min(max(c.y, 0), B.dim[1]);
+    c.z = min(max(c.z, 0), B.dim[2]);
+    return ((uint32_t)(c.z >> 3) * K.nb[1] + (c.y >> 3)) * K.nb[0] + (c.x >> 3);
+}
+
+// Further samples (in the direction of `rate`, cells per sample) certain to
+// stay in the bricks within `reach` of the one that holds cell c.
+__device__ __forceinline__ int samples_inside(const BrickCell &c, const float3 &inv, int reach) {
+    float t = 4096.0f;
+    const int b[3] = {c.x >> 3, c.y >> 3, c.z >> 3};
+    const float p[3] = {c.x + c.wx, c.y + c.wy, c.z + c.wz};
+    const float iv[3] = {inv.x, inv.y, inv.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float lo = (float)((b[k] - reach) * 8), hi = (float)((b[k] + reach + 1) * 8);
+        const float room = iv[k] > 0.0f ? hi - kDvrExitMargin - p[k] : lo + kDvrExitMargin - p[k];
+        if (iv[k] != 0.0f) t = fminf(t, room * iv[k]);
+    }
+    return t > 0.0f ? (int)t : 0;
+}
+
+// Samples per cell along each axis (0: the ray does not move along it).
+__device__ __forceinline__ float3 inverse_rate(const DvrBatch &B, const Ray &r, float step) {
+    const float x = r.dx * step * B.fdim[0], y = r.dy * step * B.fdim[1], z = r.dz * step * B.fdim[2];
+    return make_float3(fabsf(x) > 1e-6f ? 1.0f / x : 0.0f, fabsf(y) > 1e-6f ? 1.0f / y : 0.0f,
+                       fabsf(z) > 1e-6f ? 1.0f / z : 0.0f);
+}
+
+__device__ __forceinline__ float quad_trilinear(const float4 &a, const float4 &b, float wx, float wy, float wz) {
+    const float a0 = lerp(a.x, a.y, wx), a1 = lerp(a.z, a.w, wx), a2 = lerp(b.x, b.y, wx), a3 = lerp(b.z, b.w, wx);
+    return lerp(lerp(a0, a1, wy), lerp(a2, a3, wy), wz);
+}
+
+__device__ __forceinline__ float brick_trilinear(const float4 *__restrict__ q, const BrickCell &c) {
+    return quad_trilinear(__ldg(q), __ldg(q + 64), c.wx, c.wy, c.wz);
+}
+
+// The pixel and view of this thread.  A block covers 16 pixels by 2 per warp,
+// as 8x4 warp tiles whose quarter warps are 4x2 pixels.  Blocks are taken
+// from the middle of the image outwards, all views of a tile in turn, so that
+// the long rays start first.
+struct DvrPixel {
+    int x, y, view;
+};
+
+__device__ __forceinline__ int middle_out(int i, int n) {
+    const int m = (n - 1) >> 1;          // m, m + 1, m - 1, m + 2, ...
+    return m + ((i & 1) ? (i + 1) >> 1 : -(i >> 1));
+}
+
+__device__ __forceinline__ DvrPixel dvr_pixel(const DvrBatch &B, int views) {
+    const int h = blockDim.x >> 4, tx = (B.W + 15) >> 4, ty = (B.H + h - 1) / h;
+    const int t = blockIdx.x / views, row = t / tx, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    DvrPixel p;
+    p.view = blockIdx.x - t * views;
+    p.x = middle_out(t - row * tx, tx) * 16 + (warp & 1) * 8 + (lane & 3) + ((lane >> 2) & 4);
+    p.y = middle_out(row, ty) * h + (warp >> 1) * 4 + ((lane >> 2) & 3);
+    return p;
+}
+
+// Forward over bricks: the samples, their order and every operation on them
+// are k_dvr_forward's, without those that change nothing.
+constexpr int kForwardThreads = 128;
+
+template <int kAhead>
+__global__ void __launch_bounds__(kForwardThreads) k_dvr_forward_bricks(const __grid_constant__ DvrBatch B,
+                                                            const __grid_constant__ DvrBricks K, int views,
+                                                            const float4 *__restrict__ lut_g,
+                                                            float *__restrict__ images, float *__restrict__ trans,
+                                                            float *__restrict__ work) {
+    extern __shared__ float4 sm[];
+    float4 *L = sm, *D = sm + B.lut_len;
+    load_lut(lut_g, L, D, B.lut_len);
+    __syncthreads();
+    const DvrPixel px = dvr_pixel(B, views);
+    const DvrView &V = B.v[px.view];
+    const int x = px.x, y = px.y;
+    if (x >= B.W || y >= B.H) return;
+    const size_t npix = (size_t)B.W * B.H, pix = (size_t)y * B.W + x;
+    float *wk = work ? work + V.work_off : nullptr;
+    const int cmask = (1 << V.ckpt_shift) - 1;
+    float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
+    const Ray r = make_ray(B, V, x, y);
+    const float3 inv = inverse_rate(B, r, V.step);
+    // a threshold above 1 ends every ray at its first sample
+    const bool may_skip = !(T < V.t_min);
+    int i = 0, look = 0;                 // look: first sample whose brick is not known
+    const float4 *brick = K.quads;
+    bool more = r.n > 0;
+    while (more) {
+        bool sample = true;
+        if (i >= look) {
+            BrickCell c = brick_cell(B, r, V.step, (float)i);
+            const uint32_t b = brick_of(B, K, c);
+            const int d = K.dist[b];
+            look = min(i + 1 + samples_inside(c, inv, max(d - 1, 0)), r.n);
+            brick = K.quads + (size_t)b * kDvrBrickQuads;
+            if (d > 0) {
+                sample = false;
+                if (may_skip) {
+                    // (a transmittance that is not finite turns 0 * T, and with
+                    // it the colour, to NaN)
+                    if (!(fabsf(T) <= FLT_MAX)) cr = cg = cb = T * 0.0f;
+                    if (wk)
+                        for (int j = (i + cmask) & ~cmask; j < look; j += cmask + 1)
+                            wk[(size_t)(j >> V.ckpt_shift) * npix + pix] = T;
+                    i = look;
+                    more = i < r.n;
+                } else {
+                    if (wk) wk[pix] = T;
+                    i = 1;
+                    more = false;
+                }
+            }
+        }
+        if (sample) {
+            // the loads of up to kAhead samples of the brick, then their
+            // compositing in order
+            const int m = min(look - i, kAhead);
+            BrickCell c[kAhead];
+            float4 qa[kAhead], qb[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                c[k] = brick_cell(B, r, V.step, (float)(i + k));
+                const float4 *q = brick + quad_offset(c[k].x & 7, c[k].y & 7, c[k].z & 7);
+                if (k < m) {
+                    qa[k] = __ldg(q);
+                    qb[k] = __ldg(q + 64);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                if (k < m && more) {
+                    if (wk && (i & cmask) == 0) wk[(size_t)(i >> V.ckpt_shift) * npix + pix] = T;
+                    const float4 q = lut_value(L, D, lut_cell(quad_trilinear(qa[k], qb[k], c[k].wx, c[k].wy, c[k].wz), B.lut_len));
+                    const float wgt = T * q.w;
+                    cr = __fmaf_rn(wgt, q.x, cr);
+                    cg = __fmaf_rn(wgt, q.y, cg);
+                    cb = __fmaf_rn(wgt, q.z, cb);
+                    T *= (1.0f - q.w);
+                    ++i;
+                    more = i < r.n && !(T < V.t_min);
+                }
+            }
+        }
+    }
+    const size_t o = (size_t)px.view * npix + pix;
+    images[3 * o + 0] = cr;
+    images[3 * o + 1] = cg;
+    images[3 * o + 2] = cb;
+    trans[o] = T;
+    if (wk) {
+        reinterpret_cast<int *>(wk + (size_t)V.max_ckpt * npix)[pix] = i;   // samples taken
+        wk[(size_t)(V.max_ckpt + 1) * npix + pix] = T;                      // transmittance after them
+    }
+}
+
+// The LUT gradient of one ray.  Its colour part is T_i a_i times the pixel's
+// gradient, so a LUT cell needs four sums: (w0, w1) x (T a, dL/da).  They are
+// kept per lane in shared memory for a window of kWin cells about the values
+// the ray meets (noise about a tissue value stays inside it), so a sample
+// costs one 16-byte read and write without a conflict, and the block's bins
+// are touched only when a ray leaves its window.
+constexpr int kWin = 6;
+constexpr int kBackThreads = 128;
+
+__device__ __forceinline__ void bin_add(float *bins, int n, int k, float gr, float gg, float gb, const float4 &a) {
+    if (a.x != 0.0f) {
+        atomicAdd(&bins[4 * k + 0], gr * a.x);
+        atomicAdd(&bins[4 * k + 1], gg * a.x);
+        atomicAdd(&bins[4 * k + 2], gb * a.x);
+    }
+    if (a.z != 0.0f) atomicAdd(&bins[4 * k + 3], a.z);
+    if (k + 1 < n) {
+        if (a.y != 0.0f) {
+            atomicAdd(&bins[4 * k + 4], gr * a.y);
+            atomicAdd(&bins[4 * k + 5], gg * a.y);
+            atomicAdd(&bins[4 * k + 6], gb * a.y);
+        }
+        if (a.w != 0.0f) atomicAdd(&bins[4 * k + 7], a.w);
+    }
+}
+
+// The voxel sums of a cell: one 16-byte reduction per plane.
+__device__ __forceinline__ void flush_quads(float4 *g, uint32_t cell, const float (&v)[8]) {
+    if (cell == 0xffffffffu) return;
+    float4 *p = g + cell;
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :: "l"(p + 64), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
+// Backward over bricks: k_dvr_backward's reverse march; the lanes of a warp do
+// not wait for one another.  Of the colour behind a sample only its product
+// with the pixel's gradient, U . g, is needed: one recurrence instead of three.
+// The blocks' LUT sums are added up in double: thousands of blocks add to the
+// same few entries, and in fp32 that order-dependent sum was the largest
+// error of the LUT gradient (6e-7 relative, 1.6e-6 at worst).
+// 72-80 registers and 24 KB of shared memory at 256 LUT entries: six blocks per
+// SM (seven spill and leave too little L1: 1.45 -> 1.85 ms on 256^3, eight
+// views of 256^2; five: 1.52).  The next sample's loads are issued before a
+// sample is summed.  Tried and left: four lanes per ray (2.26 ms; forward 1.14
+// against 0.64: the brick look-ups are then made by every lane).
+template <bool VOLGRAD>
+__global__ void __launch_bounds__(kBackThreads, 6)
+k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant__ DvrBricks K, int views,
+                      const float4 *__restrict__ lut_g, const float *__restrict__ work,
+                      const float *__restrict__ grad_images, double *__restrict__ lut_sums,
+                      float *__restrict__ grad_vol) {
+    extern __shared__ float4 sm[];
+    const int n = B.lut_len, tid = threadIdx.x;
+    float4 *L = sm, *D = sm + n;
+    float4 *win = sm + 2 * n + tid;      // [kWin][kBackThreads]
+    float *bins = reinterpret_cast<float *>(sm + 2 * n + kWin * kBackThreads);
+    load_lut(lut_g, L, D, n);
+    for (int i = tid; i < 4 * n; i += kBackThreads) bins[i] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kWin; ++k) win[k * kBackThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+
+    const DvrPixel px = dvr_pixel(B, views);
+    const DvrView &V = B.v[px.view];
+    const bool in_image = px.x < B.W && px.y < B.H;
+    const size_t npix = (size_t)B.W * B.H, pix = in_image ? (size_t)px.y * B.W + px.x : 0;
+    const float *wk = work + V.work_off;
+    const size_t o = (size_t)px.view * npix + pix;
+    float gr = 0.f, gg = 0.f, gb = 0.f, T = 0.f;
+    int ns = 0;
+    if (in_image) {
+        gr = grad_images[3 * o];
+        gg = grad_images[3 * o + 1];
+        gb = grad_images[3 * o + 2];
+        ns = reinterpret_cast<const int *>(wk + (size_t)V.max_ckpt * npix)[pix];
+        T = wk[(size_t)(V.max_ckpt + 1) * npix + pix];
+        // (a gradient that is not finite spreads to every cell and voxel the
+        // ray meets, zero terms too: k_dvr_backward takes those rays)
+        if ((gr == 0.0f && gg == 0.0f && gb == 0.0f) || !gradient_finite(gr, gg, gb)) ns = 0;
+    }
+    const Ray r = make_ray(B, V, px.x, px.y);
+    float3 inv = inverse_rate(B, r, V.step);
+    inv = make_float3(-inv.x, -inv.y, -inv.z);
+    const int cmask = (1 << V.ckpt_shift) - 1;
+    float U = 0.0f;                      // U . g
+    int wbase = 0;                       // first LUT cell of the window
+    unsigned used = 0u;                  // its cells that hold a sum
+    uint32_t cell = 0xffffffffu;         // quad of the voxel sums (none yet)
+    float va[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) va[c] = 0.0f;
+    uint32_t brick = 0;
+    bool flat = false;
+    float flat_value = 0.0f;
+    int look = ns;                       // samples below `look` lie in bricks not known yet
+    int i = ns - 1;
+    uint32_t at = 0;                     // quad of sample i, its weights and values
+    float wx = 0.f, wy = 0.f, wz = 0.f;
+    float4 qa = make_float4(0.f, 0.f, 0.f, 0.f), qb = qa;
+    while (i >= 0) {
+        int count = 1;                   // samples this step stands for
+        if (i < look) {
+            BrickCell c = brick_cell(B, r, V.step, (float)i);
+            const uint32_t b = brick_of(B, K, c);
+            const int d = K.dist[b];
+            flat = d > 0;
+            look = max(i - samples_inside(c, inv, max(d - 1, 0)), 0);
+            brick = b * kDvrBrickQuads;
+            wx = c.wx;
+            wy = c.wy;
+            wz = c.wz;
+            if (flat) {
+                flat_value = K.flat[b];
+                count = i - look + 1;
+            } else {
+                at = brick + quad_offset(c.x & 7, c.y & 7, c.z & 7);
+                qa = __ldg(K.quads + at);
+                qb = __ldg(K.quads + at + 64);
+            }
+        }
+        const float cwx = wx, cwy = wy, cwz = wz;
+        const uint32_t cat = at;
+        const LutCell h = lut_cell(flat ? flat_value : quad_trilinear(qa, qb, wx, wy, wz), n);
+        if (!flat && i > look) {
+            // the next sample's voxels are on their way while this one is summed
+            const BrickCell c = brick_cell(B, r, V.step, (float)(i - 1));
+            at = brick + quad_offset(c.x & 7, c.y & 7, c.z & 7);
+            wx = c.wx;
+            wy = c.wy;
+            wz = c.wz;
+            qa = __ldg(K.quads + at);
+            qb = __ldg(K.quads + at + 64);
+        }
+        const float4 q = lut_value(L, D, h);
+        const float d = 1.0f - q.w;
+        const int ck = i & ~cmask;       // the last checkpoint at or before sample i
+        if (ck > i - count) {
+            T = wk[(size_t)(ck >> V.ckpt_shift) * npix + pix];
+        } else if (d == 0.0f) {
+            T = wk[(size_t)(ck >> V.ckpt_shift) * npix + pix];
+            for (int j = ck; j < i; ++j) {
+                BrickCell e = brick_cell(B, r, V.step, (float)j);
+                const uint32_t b = brick_of(B, K, e);
+                if (K.dist[b] != 0) continue;          // alpha 0
+                const uint32_t qe = b * kDvrBrickQuads + quad_offset(e.x & 7, e.y & 7, e.z & 7);
+                T *= 1.0f - lut_value(L, D, lut_cell(brick_trilinear(K.quads + qe, e), n)).w;
+            }
+        } else if (d != 1.0f) {
+            T = T / d;
+        }
+        const float ta = T * q.w, p = gr * q.x + gg * q.y + gb * q.z;
+        const float d_a = T * (p - U);
+        U = q.w * p + d * U;
+        // LUT sums
+        int slot = h.k - wbase;
+        if ((unsigned)slot >= (unsigned)kWin) {
+            while (used) {
+                const int u = __ffs(used) - 1;
+                used &= used - 1u;
+                bin_add(bins, n, wbase + u, gr, gg, gb, win[u * kBackThreads]);
+                win[u * kBackThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            wbase = max(h.k - kWin / 2, 0);
+            slot = h.k - wbase;
+        }
+        used |= 1u << slot;
+        {
+            const float w1 = h.w, w0 = 1.0f - h.w, da = (float)count * d_a;
+            float4 a = win[slot * kBackThreads];
+            a.x += w0 * ta;
+            a.y += w1 * ta;
+            a.z += w0 * da;
+            a.w += w1 * da;
+            win[slot * kBackThreads] = a;
+        }
+        // voxel sums
+        if (VOLGRAD && h.inside) {
+            const float4 dd = D[h.k];
+            const float ds = (float)n * (ta * (gr * dd.x + gg * dd.y + gb * dd.z) + d_a * dd.w);
+            if (ds != 0.0f) {
+                const float y0z0 = (1.0f - cwy) * (1.0f - cwz) * ds, y1z0 = cwy * (1.0f - cwz) * ds;
+                const float y0z1 = (1.0f - cwy) * cwz * ds, y1z1 = cwy * cwz * ds;
+                const float x0 = 1.0f - cwx, x1 = cwx;
+                if (flat || !(fabsf(ds) <= FLT_MAX)) {
+                    // not finite: to the voxels themselves, whatever the brick holds
+                    const float v[8] = {x0 * y0z0, x1 * y0z0, x0 * y1z0, x1 * y1z0, x0 * y0z1, x1 * y0z1, x0 * y1z1, x1 * y1z1};
+                    for (int j = i; j > i - count; --j) {
+                        const BrickCell c = brick_cell(B, r, V.step, (float)j);
+                        flush_vol(grad_vol, B, c.x - 1, c.y - 1, c.z - 1, v);
+                    }
+                } else {
+                    if (cat != cell) {
+                        flush_quads(K.gquads, cell, va);
+                        cell = cat;
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) va[k] = 0.0f;
+                    }
+                    va[0] += x0 * y0z0;
+                    va[1] += x1 * y0z0;
+                    va[2] += x0 * y1z0;
+                    va[3] += x1 * y1z0;
+                    va[4] += x0 * y0z1;
+                    va[5] += x1 * y0z1;
+                    va[6] += x0 * y1z1;
+                    va[7] += x1 * y1z1;
+                }
+            }
+        }
+        i -= count;
+    }
+    if (VOLGRAD) flush_quads(K.gquads, cell, va);
+    __syncwarp();
+#pragma unroll 1
+    for (int u = 0; u < kWin; ++u) {
+        const bool has = (used >> u) & 1u;
+        const float4 a = win[u * kBackThreads];
+        const float4 a0 = make_float4(gr * a.x, gg * a.x, gb * a.x, a.z), a1 = make_float4(gr * a.y, gg * a.y, gb * a.y, a.w);
+        flush_lut_warp(bins, n, has, wbase + u, a0, a1);
+    }
+    __syncthreads();
+    for (int k = tid; k < 4 * n; k += kBackThreads) {
+        const float v = bins[k];
+        if (v != 0.0f) atomicAdd(&lut_sums[k], (double)v);
+    }
+}
+
+__global__ void k_dvr_lut_add(int n, const double *__restrict__ sums, float *__restrict__ grad_lut) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && sums[i] != 0.0) atomicAdd(&grad_lut[i], (float)sums[i]);
+}
+
+// ---------------------------------------------------------------------------
 // host side
 
 // Checkpoint spacing of a view: 16 samples, doubled until at most 512
@@ -542,6 +1143,110 @@ static void fill_batch(const mk_dvr_params *views, int first, int count, size_t 
     }
 }
 
+// Scratch of the bricked path: the bricks' quads (twice with voxel
+// gradients), then flat values, LUT gradient sums, need bytes and the distance
+// map and its intermediate.
+struct BrickLayout {
+    int nb[3];
+    size_t n;                            // bricks
+    size_t gquads, flat, lut, needed, tmp, dist, bytes;
+};
+
+static BrickLayout brick_layout(const int dims[3], bool gradients) {
+    BrickLayout l;
+    for (int k = 0; k < 3; ++k) l.nb[k] = dims[k] / 8 + 1;       // dims + 1 cells
+    l.n = (size_t)l.nb[0] * l.nb[1] * l.nb[2];
+    const size_t quads = l.n * kDvrBrickQuads * sizeof(float4), pad = (l.n + 255) & ~(size_t)255;
+    l.gquads = quads;
+    l.flat = quads * (gradients ? 2 : 1);
+    l.lut = l.flat + 4 * pad;
+    l.needed = l.lut + 4 * kDvrMaxLut * sizeof(double);
+    l.tmp = l.needed + pad;
+    l.dist = l.tmp + pad;
+    l.bytes = l.dist + pad;
+    return l;
+}
+
+// Whether these views gain from bricks, and may use them.  A view has about
+// W * H * 0.5 / step samples.  Measured at a quarter of a sample per voxel (one
+// view of 128^2, 256^3, plain / bricks): forward 426 / 122 us where most is
+// transparent, 426 / 377 us where all is visible; backward 1256 / 734 and 1369
+// / 1312 us.  At a sixteenth the visible case turns (backward 1245 / 1401 us).
+// The exit model of a ray (linear in the sample number) holds to a few hundredths of a
+// cell while a unit of the ray parameter is at most 3e4 cells along an axis;
+// quads are addressed with 32 bits.
+constexpr double kDvrSamplesPerVoxel = 0.25;
+constexpr double kDvrMaxCellsPerUnit = 3.0e4;
+
+static bool use_bricks(const mk_dvr_params *views, int nviews) {
+    const mk_dvr_params &a = views[0];
+    double samples = 0.0;
+    for (int i = 0; i < nviews; ++i) {
+        const mk_dvr_params &p = views[i];
+        samples += (double)p.width * p.height * 0.5 / p.step;
+        for (int k = 0; k < 3; ++k) {
+            const double unit = fabs((double)p.transform[3 * k + 1] * p.scale * p.max_len_spacing[k]) * a.dims[k];
+            if (!(unit <= kDvrMaxCellsPerUnit)) return false;
+        }
+    }
+    for (int k = 0; k < 3; ++k)
+        if (a.dims[k] > 4096) return false;
+    const BrickLayout l = brick_layout(a.dims, false);
+    if (l.nb[1] > 65535 || l.nb[2] > 65535 || l.n * kDvrBrickQuads >= 0xffffffffull) return false;
+    return samples >= kDvrSamplesPerVoxel * a.dims[0] * a.dims[1] * (double)a.dims[2];
+}
+
+// Build the bricks of `volume` under `lut` in `scratch`, and their distances.
+template <bool BACKWARD>
+static int build_bricks(const mk_dvr_params &p, const float *volume, const float *lut, void *scratch, bool gradients,
+                        DvrBricks &K, cudaStream_t s) {
+    const BrickLayout l = brick_layout(p.dims, gradients);
+    char *base = static_cast<char *>(scratch);
+    float4 *quads = reinterpret_cast<float4 *>(base);
+    float4 *gquads = gradients ? reinterpret_cast<float4 *>(base + l.gquads) : nullptr;
+    float *flat = reinterpret_cast<float *>(base + l.flat);
+    uint8_t *needed = reinterpret_cast<uint8_t *>(base + l.needed);
+    uint8_t *dist = reinterpret_cast<uint8_t *>(base + l.dist);
+    k_dvr_build<BACKWARD><<<dim3((l.nb[0] + 3) / 4, l.nb[1], l.nb[2]), 256, 0, s>>>(
+        p.dims[0], p.dims[1], p.dims[2], l.nb[0], volume, reinterpret_cast<const float4 *>(lut), p.lut_len, quads, gquads, needed,
+        flat);
+    MK_CUDA_TRY(cudaGetLastError());
+    for (int k = 0; k < 3; ++k) K.nb[k] = l.nb[k];
+    K.quads = quads;
+    K.gquads = gquads;
+    K.dist = dist;
+    K.flat = flat;
+    return launch_brick_distance(needed, l.nb[0], l.nb[1], l.nb[2], reinterpret_cast<uint8_t *>(base + l.tmp), dist, s);
+}
+
+// Blocks of `threads` threads over the views of a batch (dvr_pixel).
+static unsigned dvr_blocks(const DvrBatch &B, int views, int threads) {
+    const unsigned h = threads / 16;
+    return ((B.W + 15) / 16) * ((B.H + h - 1) / h) * (unsigned)views;
+}
+
+// Samples whose loads a ray has in flight: four where the launch is too small
+// to fill the SMs and the longest rays set its time (one view of 321x243:
+// 107 us, against 118 with two and 150 with one), two where there are rays
+// enough (eight views of 256^2: 638 us, against 670 with four, whose registers
+// cost resident warps, and 686 with one).  The line: about 2000 rays per SM.
+constexpr long long kDvrManyRays = 300000;
+
+static void launch_forward_bricks(const DvrBatch &B, const DvrBricks &K, int views, const float4 *lut, float *images,
+                                  float *trans, float *work, size_t smem, cudaStream_t s) {
+    const unsigned grid = dvr_blocks(B, views, kForwardThreads);
+    if ((long long)B.W * B.H * views >= kDvrManyRays)
+        k_dvr_forward_bricks<2><<<grid, kForwardThreads, smem, s>>>(B, K, views, lut, images, trans, work);
+    else
+        k_dvr_forward_bricks<4><<<grid, kForwardThreads, smem, s>>>(B, K, views, lut, images, trans, work);
+}
+
+// Scratch the caller gave, if it is enough and aligned for these views.
+static bool bricks_fit(const mk_dvr_params *views, int nviews, bool gradients, const void *scratch, size_t bytes) {
+    return scratch && (reinterpret_cast<uintptr_t>(scratch) & 255) == 0 && use_bricks(views, nviews) &&
+           bytes >= brick_layout(views[0].dims, gradients).bytes;
+}
+
 }  // namespace mk
 
 using namespace mk;
@@ -559,8 +1264,20 @@ extern "C" int mk_dvr_workspace_floats(const mk_dvr_params *views, int nviews, s
     return MK_OK;
 }
 
-extern "C" int mk_dvr_forward(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
-                              float *images, float *transmittance, float *workspace, void *stream) {
+extern "C" int mk_dvr_scratch_bytes(const mk_dvr_params *views, int nviews, int gradients, size_t *bytes) {
+    if (!bytes) {
+        set_last_error("mk_dvr_scratch_bytes: null argument");
+        return MK_ERR_INVALID_ARGUMENT;
+    }
+    int rc = check_views(views, nviews);
+    if (rc != MK_OK) return rc;
+    *bytes = use_bricks(views, nviews) ? brick_layout(views[0].dims, gradients != 0).bytes : 0;
+    return MK_OK;
+}
+
+extern "C" int mk_dvr_forward_scratch(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
+                                      float *images, float *transmittance, float *workspace, void *scratch,
+                                      size_t scratch_bytes, void *stream) {
     if (!volume || !lut || !images || !transmittance) {
         set_last_error("mk_dvr_forward: null argument");
         return MK_ERR_INVALID_ARGUMENT;
@@ -570,7 +1287,14 @@ extern "C" int mk_dvr_forward(const mk_dvr_params *views, int nviews, const floa
     cudaStream_t s = (cudaStream_t)stream;
     const size_t npix = (size_t)views[0].width * views[0].height;
     const size_t smem = 2 * (size_t)views[0].lut_len * sizeof(float4);
-    MK_CUDA_TRY(cudaFuncSetAttribute(k_dvr_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const bool bricks = bricks_fit(views, nviews, false, scratch, scratch_bytes);
+    DvrBricks K = {};
+    if (bricks) {
+        rc = build_bricks<false>(views[0], volume, lut, scratch, false, K, s);
+        if (rc != MK_OK) return rc;
+    } else {
+        MK_CUDA_TRY(cudaFuncSetAttribute(k_dvr_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
     size_t off = 0;
     DvrBatch B;
     for (int first = 0; first < nviews; first += kDvrViewsPerLaunch) {
@@ -578,17 +1302,23 @@ extern "C" int mk_dvr_forward(const mk_dvr_params *views, int nviews, const floa
         fill_batch(views, first, count, off, B);
         for (int i = 0; i < count; ++i) off += view_floats(views[first + i]);
         dim3 grid((B.W + 31) / 32, (B.H + 7) / 8, count);
-        k_dvr_forward<<<grid, 256, smem, s>>>(B, volume, reinterpret_cast<const float4 *>(lut),
-                                              images + (size_t)first * npix * 3, transmittance + (size_t)first * npix,
-                                              workspace);
+        const float4 *l4 = reinterpret_cast<const float4 *>(lut);
+        float *im = images + (size_t)first * npix * 3, *tr = transmittance + (size_t)first * npix;
+        if (bricks) launch_forward_bricks(B, K, count, l4, im, tr, workspace, smem, s);
+        else k_dvr_forward<<<grid, 256, smem, s>>>(B, volume, l4, im, tr, workspace);
         MK_CUDA_TRY(cudaGetLastError());
     }
     return MK_OK;
 }
 
-extern "C" int mk_dvr_backward(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
-                               const float *workspace, const float *grad_images, float *grad_lut,
-                               float *grad_volume, void *stream) {
+extern "C" int mk_dvr_forward(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
+                              float *images, float *transmittance, float *workspace, void *stream) {
+    return mk_dvr_forward_scratch(views, nviews, volume, lut, images, transmittance, workspace, nullptr, 0, stream);
+}
+
+extern "C" int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
+                                       const float *workspace, const float *grad_images, float *grad_lut,
+                                       float *grad_volume, void *scratch, size_t scratch_bytes, void *stream) {
     if (!volume || !lut || !workspace || !grad_images || !grad_lut) {
         set_last_error("mk_dvr_backward: null argument");
         return MK_ERR_INVALID_ARGUMENT;
@@ -597,9 +1327,23 @@ extern "C" int mk_dvr_backward(const mk_dvr_params *views, int nviews, const flo
     if (rc != MK_OK) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t npix = (size_t)views[0].width * views[0].height;
-    const size_t smem = 3 * (size_t)views[0].lut_len * sizeof(float4);
-    auto kern = grad_volume ? k_dvr_backward<true> : k_dvr_backward<false>;
-    MK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const bool bricks = bricks_fit(views, nviews, grad_volume != nullptr, scratch, scratch_bytes);
+    const size_t smem = 3 * (size_t)views[0].lut_len * sizeof(float4), smem_b = smem + kWin * kBackThreads * sizeof(float4);
+    DvrBricks K = {};
+    double *lut_sums = nullptr;
+    auto kern = grad_volume ? k_dvr_backward<true, false> : k_dvr_backward<false, false>;
+    auto kern_odd = grad_volume ? k_dvr_backward<true, true> : k_dvr_backward<false, true>;
+    auto kern_b = grad_volume ? k_dvr_backward_bricks<true> : k_dvr_backward_bricks<false>;
+    if (bricks) {
+        MK_CUDA_TRY(cudaFuncSetAttribute(kern_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
+        MK_CUDA_TRY(cudaFuncSetAttribute(kern_odd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        lut_sums = reinterpret_cast<double *>(static_cast<char *>(scratch) + brick_layout(views[0].dims, grad_volume != nullptr).lut);
+        MK_CUDA_TRY(cudaMemsetAsync(lut_sums, 0, 4 * views[0].lut_len * sizeof(double), s));
+        rc = build_bricks<true>(views[0], volume, lut, scratch, grad_volume != nullptr, K, s);
+        if (rc != MK_OK) return rc;
+    } else {
+        MK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
     size_t off = 0;
     DvrBatch B;
     for (int first = 0; first < nviews; first += kDvrViewsPerLaunch) {
@@ -607,9 +1351,36 @@ extern "C" int mk_dvr_backward(const mk_dvr_params *views, int nviews, const flo
         fill_batch(views, first, count, off, B);
         for (int i = 0; i < count; ++i) off += view_floats(views[first + i]);
         dim3 grid((B.W + 15) / 16, (B.H + 7) / 8, count);
-        kern<<<grid, 128, smem, s>>>(B, volume, reinterpret_cast<const float4 *>(lut), workspace,
-                                     grad_images + (size_t)first * npix * 3, grad_lut, grad_volume);
+        const float4 *l4 = reinterpret_cast<const float4 *>(lut);
+        const float *gi = grad_images + (size_t)first * npix * 3;
+        if (bricks) {
+            kern_b<<<dvr_blocks(B, count, kBackThreads), kBackThreads, smem_b, s>>>(B, K, count, l4, workspace, gi, lut_sums,
+                                                                                  grad_volume);
+            MK_CUDA_TRY(cudaGetLastError());
+            kern_odd<<<grid, 128, smem, s>>>(B, volume, l4, workspace, gi, grad_lut, grad_volume);
+        } else {
+            kern<<<grid, 128, smem, s>>>(B, volume, l4, workspace, gi, grad_lut, grad_volume);
+        }
+        MK_CUDA_TRY(cudaGetLastError());
+    }
+    if (bricks) {
+        const int n = 4 * views[0].lut_len;
+        k_dvr_lut_add<<<(n + 255) / 256, 256, 0, s>>>(n, lut_sums, grad_lut);
+        MK_CUDA_TRY(cudaGetLastError());
+    }
+    if (bricks && grad_volume) {
+        const mk_dvr_params &p = views[0];
+        const BrickLayout l = brick_layout(p.dims, true);
+        k_dvr_fold<<<dim3(l.nb[0], l.nb[1], l.nb[2]), 256, 0, s>>>(
+            p.dims[0], p.dims[1], p.dims[2], K.gquads, reinterpret_cast<const uint8_t *>(scratch) + l.needed, grad_volume);
         MK_CUDA_TRY(cudaGetLastError());
     }
     return MK_OK;
+}
+
+extern "C" int mk_dvr_backward(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
+                               const float *workspace, const float *grad_images, float *grad_lut,
+                               float *grad_volume, void *stream) {
+    return mk_dvr_backward_scratch(views, nviews, volume, lut, workspace, grad_images, grad_lut, grad_volume, nullptr, 0,
+                                   stream);
 }

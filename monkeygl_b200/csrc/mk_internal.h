@@ -181,6 +181,11 @@ int rebuild_brick_maps(VolumeState *v, cudaStream_t s);
 // (alpha, ww, wl) rows, written to vis_bits / mip_tmax on stream s.
 int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha, const int *lut_len,
                             const float (*params)[3], uint32_t *vis_bits, float *mip_tmax, cudaStream_t s);
+// Distance map over bricks (mk_brickdist.cu): `occupied` is one byte per brick
+// (0: empty), `tmp` and `dist` one byte per brick each.
+constexpr int kMaxBrickDist = 8;
+int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, uint8_t *tmp, uint8_t *dist,
+                          cudaStream_t s);
 // Words of visibility bits / floats of MIP bounds of a volume's brick maps.
 inline size_t brick_count(const VolumeState *v) { return (size_t)v->nb[0] * v->nb[1] * v->nb[2]; }
 int finish_output(VolumeState *v, void *out, size_t bytes, int out_on_device, cudaStream_t s);

@@ -78,6 +78,18 @@ def workspace_floats(views) -> int:
 def _torch_function():
     import torch
 
+    def scratch(arr, nv, gradients, device):
+        """Scratch for one call on the current stream (which the caching
+        allocator hands the memory back to), or none if it does not fit."""
+        n = C.c_size_t(0)
+        _check(_lib().mk_dvr_scratch_bytes(arr, nv, int(gradients), C.byref(n)), "mk_dvr_scratch_bytes")
+        if n.value == 0:
+            return None, 0
+        try:
+            return torch.empty(n.value, dtype=torch.uint8, device=device), n.value
+        except torch.cuda.OutOfMemoryError:
+            return None, 0
+
     class VolumeRender(torch.autograd.Function):
         @staticmethod
         def forward(ctx, volume, lut, views):
@@ -99,8 +111,9 @@ def _torch_function():
             work = None
             if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
                 work = torch.empty(workspace_floats(arr), dtype=torch.float32, device=volume.device)
-            _check(L.mk_dvr_forward(arr, nv, _ptr(volume), _ptr(lut), _ptr(images), _ptr(trans), _ptr(work),
-                                    stream), "mk_dvr_forward")
+            tmp, tmp_bytes = scratch(arr, nv, False, volume.device)
+            _check(L.mk_dvr_forward_scratch(arr, nv, _ptr(volume), _ptr(lut), _ptr(images), _ptr(trans), _ptr(work),
+                                            _ptr(tmp), tmp_bytes, stream), "mk_dvr_forward")
             ctx.views = arr
             ctx.work = work
             ctx.save_for_backward(volume, lut)
@@ -114,8 +127,10 @@ def _torch_function():
             grad_lut = torch.zeros_like(lut)
             grad_vol = torch.zeros_like(volume) if ctx.needs_input_grad[0] else None
             g = grad_images.contiguous().float()
-            _check(L.mk_dvr_backward(ctx.views, len(ctx.views), _ptr(volume), _ptr(lut), _ptr(ctx.work), _ptr(g),
-                                     _ptr(grad_lut), _ptr(grad_vol), stream), "mk_dvr_backward")
+            tmp, tmp_bytes = scratch(ctx.views, len(ctx.views), grad_vol is not None, volume.device)
+            _check(L.mk_dvr_backward_scratch(ctx.views, len(ctx.views), _ptr(volume), _ptr(lut), _ptr(ctx.work), _ptr(g),
+                                             _ptr(grad_lut), _ptr(grad_vol), _ptr(tmp), tmp_bytes, stream),
+                   "mk_dvr_backward")
             return grad_vol, (grad_lut if ctx.needs_input_grad[1] else None), None
 
     return VolumeRender
