@@ -52,9 +52,9 @@ __global__ void __launch_bounds__(256) k_brick_distance_z(const uint8_t *__restr
     dist[i] = (uint8_t)line_distance(in + i, nxy, (int)(i / nxy), nbz);
 }
 
-// Slices too large for shared memory: every empty brick is its own step.
-__global__ void __launch_bounds__(256) k_brick_distance_one(const uint8_t *__restrict__ occupied, size_t n,
-                                                            uint8_t *__restrict__ dist) {
+// Every empty brick is its own step (also for slices too large for shared
+// memory).
+__global__ void __launch_bounds__(256) k_brick_distance_one(const uint8_t *occupied, size_t n, uint8_t *dist) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dist[i] = occupied[i] ? 0 : 1;
 }
@@ -63,11 +63,11 @@ constexpr size_t kMaxSliceSmem = 200 * 1024;
 
 }  // namespace
 
-int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, uint8_t *tmp, uint8_t *dist,
+int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, bool one, uint8_t *tmp, uint8_t *dist,
                           cudaStream_t s) {
     const size_t nxy = (size_t)nbx * nby, n = nxy * nbz;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (2 * nxy > kMaxSliceSmem) {
+    if (one || 2 * nxy > kMaxSliceSmem) {
         k_brick_distance_one<<<blocks, 256, 0, s>>>(occupied, n, dist);
     } else {
         if (2 * nxy > 48 * 1024)

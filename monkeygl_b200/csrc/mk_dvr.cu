@@ -1216,7 +1216,7 @@ static int build_bricks(const mk_dvr_params &p, const float *volume, const float
     K.gquads = gquads;
     K.dist = dist;
     K.flat = flat;
-    return launch_brick_distance(needed, l.nb[0], l.nb[1], l.nb[2], reinterpret_cast<uint8_t *>(base + l.tmp), dist, s);
+    return launch_brick_distance(needed, l.nb[0], l.nb[1], l.nb[2], false, reinterpret_cast<uint8_t *>(base + l.tmp), dist, s);
 }
 
 // Blocks of `threads` threads over the views of a batch (dvr_pixel).

@@ -37,7 +37,8 @@ struct LabelTable {
 
 // Per-frame view of the brick maps handed to the ray-casting kernels.
 struct BrickView {
-    const uint32_t *visible_bits;   // VR: 1 = some sample may have alpha > kEmptyAlpha
+    const uint8_t *dist;            // VR: 0 = some sample may have alpha > kEmptyAlpha, else the
+                                    // distance to the next such brick (mk_brickdist.cu)
     const float *mip_tmax;          // MIP: upper bound of the windowed value over labels with alpha > 0
     const short2 *minmax;           // raw voxel min/max of the footprint
     int nbx, nby, nbz;
@@ -81,7 +82,8 @@ struct VolumeState {
     int nb[3] = {0, 0, 0};
     short2 *d_minmax = nullptr;
     uint32_t *d_labels = nullptr;            // 3 words (labels 0..64) per brick
-    uint32_t *d_visible = nullptr;           // 1 bit per brick
+    uint8_t *d_dist = nullptr;               // VR distance map, a byte per brick, and its scratch
+    uint8_t *d_dist_tmp = nullptr;
     float *d_mip_tmax = nullptr;
     bool maps_dirty = true;
     uint64_t present_labels[2] = {1, 0};     // labels occurring anywhere in the mask
@@ -176,17 +178,19 @@ float float_bound_above(double c);
 int ensure_device_buffer(VolumeState *v, size_t bytes);
 int ensure_pinned_buffer(VolumeState *v, size_t bytes);
 int rebuild_brick_maps(VolumeState *v, cudaStream_t s);
-// Brick visibility bits and MIP bounds of volume v for the given per-label
-// LUT alpha columns (device pointers, nullptr = no table), LUT lengths and
-// (alpha, ww, wl) rows, written to vis_bits / mip_tmax on stream s.
+// The VR distance map (dist, with scratch tmp: a byte per brick each) and MIP
+// bounds (mip_tmax) of volume v for the given per-label LUT alpha columns
+// (device pointers, nullptr = no table), LUT lengths and (alpha, ww, wl) rows,
+// on stream s.  Either may be null.
 int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha, const int *lut_len,
-                            const float (*params)[3], uint32_t *vis_bits, float *mip_tmax, cudaStream_t s);
+                            const float (*params)[3], uint8_t *dist, uint8_t *tmp, float *mip_tmax, cudaStream_t s);
 // Distance map over bricks (mk_brickdist.cu): `occupied` is one byte per brick
-// (0: empty), `tmp` and `dist` one byte per brick each.
+// (0: empty), `tmp` and `dist` one byte per brick each; `dist` may be
+// `occupied`.  one: no distances, 1 for every empty brick.
 constexpr int kMaxBrickDist = 8;
-int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, uint8_t *tmp, uint8_t *dist,
+int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, bool one, uint8_t *tmp, uint8_t *dist,
                           cudaStream_t s);
-// Words of visibility bits / floats of MIP bounds of a volume's brick maps.
+// Bytes of the distance map / floats of MIP bounds of a volume's brick maps.
 inline size_t brick_count(const VolumeState *v) { return (size_t)v->nb[0] * v->nb[1] * v->nb[2]; }
 int finish_output(VolumeState *v, void *out, size_t bytes, int out_on_device, cudaStream_t s);
 // True for page-locked host memory the device can copy to directly.

@@ -10,6 +10,7 @@
 #pragma once
 
 #include <math.h>
+#include <string.h>
 #include <stdint.h>
 
 #if defined(__CUDACC__)
@@ -41,6 +42,32 @@ MK_HD short f2s_sat(float v) {
     if (v >= 32767.0f) return 32767;
     if (v <= -32768.0f) return -32768;
     return (short)v;
+}
+
+// a after n additions of `step`, each rounded to float, as MonkeyGL's loop
+// makes them.  Between two powers of two all floats have one spacing, so every
+// addition moves a by the same amount (after the first sum in that range: a
+// step that falls halfway between two floats is rounded to the even one, and
+// from an even one always the same way); that amount is an exact difference
+// and n times it an exact product.  Where the sum leaves the range, one
+// addition at a time.
+MK_HD float add_steps(float a, float step, int n) {
+    if (n > 4) {
+        const float a1 = a + step, a2 = a1 + step, d = (a2 + step) - a2;
+#ifdef __CUDA_ARCH__
+        const float end = __fmaf_rn((float)(n - 2), d, a2);
+        const bool same = ((__float_as_uint(a1) ^ __float_as_uint(end)) >> 23) == 0u;
+#else
+        const float end = fmaf((float)(n - 2), d, a2);
+        uint32_t u, v;
+        memcpy(&u, &a1, 4);
+        memcpy(&v, &end, 4);
+        const bool same = ((u ^ v) >> 23) == 0u;
+#endif
+        if (same) return end;
+    }
+    for (; n > 0; --n) a += step;
+    return a;
 }
 
 }  // namespace mk

@@ -18,11 +18,17 @@
 //    a table) and stops once past it.  Samples outside that interval are
 //    provably outside the VOI, where MonkeyGL only advances accuLength.
 //  * Empty-space skipping.  While the ray is at the coarse step with a small
-//    previous alpha, a sample inside a brick whose visibility bit is clear
-//    cannot composite or refine the step (its alpha is <= kEmptyAlpha), so
-//    the texture fetches are skipped; accuLength still advances by the same
-//    float additions, and runs of such samples up to the brick exit are
-//    advanced with additions only.  MIP skips bricks whose bound cannot
+//    previous alpha, a sample inside a brick that no transfer function can
+//    show cannot composite or refine the step (its alpha is <= kEmptyAlpha),
+//    so the texture fetches are skipped; accuLength still advances by the same
+//    float additions.  A byte per brick holds the distance to the next brick
+//    that can show (mk_brickdist.cu), and one step takes the ray across the
+//    whole cube of empty bricks around it, up to 64 voxels, through the
+//    schedule table or add_steps.  With a bit per brick a ray stopped at every
+//    brick face, and those visits were most of a frame's instructions:
+//    1024^2 frames of a 512x512x361 volume 389 -> 225 us (tile launch), of a
+//    labelled 512x512x1559 one 226 -> 153 us; the map costs 7 us per change
+//    of a transfer function or window.  MIP skips bricks whose bound cannot
 //    raise the running maximum and stops at 1.0 (the 8-bit output
 //    saturates); SURFACE skips bricks whose voxels are all <= 400 HU.
 //  * Warp-coherent tiles.  A 256-thread block covers a 32x8 pixel tile as
@@ -31,8 +37,8 @@
 //    stored as aligned 32-bit words.
 //  * Per-label opacity caps live in shared memory (or registers when no
 //    label needs one) instead of a 65-float local array per thread.
-//  * FP32 only: MonkeyGL's double-promoted expressions are reproduced with
-//    error-free float transformations (mk_math.h).
+//  * MonkeyGL's double-promoted expressions are evaluated in double, operation
+//    for operation (mk_math.h).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

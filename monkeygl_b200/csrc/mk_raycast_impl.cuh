@@ -199,28 +199,30 @@ __device__ __forceinline__ StepVec step_vec(const RayParams &P) {
     return S;
 }
 
-// Number of further coarse steps that stay inside brick (bx,by,bz) with a
-// 0.05-voxel margin, capped at 64.  Position p is in voxel units.  Any
-// count that keeps those samples inside the brick is valid (they are all
-// skippable); the margin covers the rounding of the linear model.
-__device__ __forceinline__ int steps_in_brick(const float3 &pv, const StepVec &sv, int ix, int iy, int iz) {
-    float t = 64.0f;
-    const float e = 0.05f;
-    const float lo[3] = {(float)((ix >> kBrickShift) << kBrickShift),
-                         (float)((iy >> kBrickShift) << kBrickShift),
-                         (float)((iz >> kBrickShift) << kBrickShift)};
+// Number of further coarse steps that stay, with a 0.05-voxel margin, inside
+// the cube of bricks within `reach` of the one that holds voxel (ix,iy,iz);
+// capped at kMaxRun.  Position p is in voxel units.  Any count that keeps those
+// samples inside the cube is valid (they are all skippable); the margin covers
+// the rounding of the linear model.
+constexpr int kMaxRun = 240;
+__device__ __forceinline__ int steps_in_brick(const float3 &pv, const StepVec &sv, int ix, int iy, int iz,
+                                              int reach = 0) {
+    float t = (float)kMaxRun;
+    const float e = 0.05f, back = (float)(reach * kBrick), width = (float)((2 * reach + 1) * kBrick);
+    const float lo[3] = {(float)((ix >> kBrickShift) << kBrickShift) - back,
+                         (float)((iy >> kBrickShift) << kBrickShift) - back,
+                         (float)((iz >> kBrickShift) << kBrickShift) - back};
     const float pp[3] = {pv.x, pv.y, pv.z};
     const float rd[3] = {sv.rdv.x, sv.rdv.y, sv.rdv.z};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        if (rd[k] > 0.0f) t = fminf(t, (lo[k] + kBrick - e - pp[k]) * rd[k]);
+        if (rd[k] > 0.0f) t = fminf(t, (lo[k] + width - e - pp[k]) * rd[k]);
         else if (rd[k] < 0.0f) t = fminf(t, (pp[k] - lo[k] - e) * -rd[k]);
     }
     return t > 0.0f ? (int)t : 0;
 }
 
-// Advance accuLength by n coarse steps: n float additions of L1, as
-// MonkeyGL's loop makes them.  While a ray has never refined its step it
+// Advance accuLength by n coarse steps of L1.  While a ray has never refined its step it
 // stays on the schedule table (a == accu[lat]), whose entry lat + n holds
 // the same sum; lat < 0 once the ray has left it.
 __device__ __forceinline__ void advance_coarse(const RayParams &P, float &a, int &lat, float step, int n) {
@@ -228,7 +230,7 @@ __device__ __forceinline__ void advance_coarse(const RayParams &P, float &a, int
         lat = min(lat + n, P.accu_len - 1);
         a = P.accu[lat];
     } else {
-        for (; n > 0; --n) a += step;
+        a = add_steps(a, step, n);
     }
 }
 
@@ -548,10 +550,7 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
                 if (kj >= 0) {
                     aj = P.accu[kj];
                 } else {
-                    // sequential additions, as the walk makes them
-#pragma unroll
-                    for (int k = 0; k < 31; ++k)
-                        if (k < jj) aj += sj;
+                    aj = add_steps(aj, sj, jj);
                 }
                 if (!(aj < P.limit) || aj > Q.a_stop) {
                     flags = kCoopEnd;
@@ -565,11 +564,11 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
                     } else {
                         bool empty = false;
                         if (P.skip && sj == L1) {
-                            const int b = brick_index(P, BV, ix, iy, iz);
-                            empty = !((BV.visible_bits[b >> 5] >> (b & 31)) & 1u);
+                            const int dist = BV.dist[brick_index(P, BV, ix, iy, iz)];
+                            empty = dist != 0;
                             if (empty) {
                                 const float3 pv = make_float3(pos.x * P.fdim[0], pos.y * P.fdim[1], pos.z * P.fdim[2]);
-                                nskip = steps_in_brick(pv, dv, ix, iy, iz);
+                                nskip = steps_in_brick(pv, dv, ix, iy, iz, dist - 1);
                                 flags |= kCoopEmpty;
                             }
                         }
@@ -953,11 +952,11 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
                     break;
                 }
                 if (P.skip && R.step == L1 && R.aPre <= 0.001f) {
-                    const int b = brick_index(P, BV, ix, iy, iz);
-                    if (!((BV.visible_bits[b >> 5] >> (b & 31)) & 1u)) {
+                    const int dist = BV.dist[brick_index(P, BV, ix, iy, iz)];
+                    if (dist != 0) {
                         R.aPre = 0.0f;
                         const float3 pv = make_float3(pos.x * P.fdim[0], pos.y * P.fdim[1], pos.z * P.fdim[2]);
-                        advance_coarse(P, R.a, R.lat, R.step, 1 + steps_in_brick(pv, dv, ix, iy, iz));
+                        advance_coarse(P, R.a, R.lat, R.step, 1 + steps_in_brick(pv, dv, ix, iy, iz, dist - 1));
                         break;
                     }
                 }

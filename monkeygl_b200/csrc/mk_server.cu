@@ -10,7 +10,7 @@
 //  * A request takes a slot: its LUTs go to the slot's 1D float4 texture
 //    arrays (same filtering as mk_volume_set_transfer_function), its label
 //    parameters and kernel parameters to the slot's descriptor, and the
-//    brick visibility / MIP bounds of its volume under its tables are built
+//    brick distance map or MIP bounds of its volume under its tables are built
 //    into the slot's maps -- the same kernel and inputs mk_render_vr uses, so
 //    the image equals mk_render_vr's for the same request.
 //  * Every step, the worker thread lists up to tiles_per_step 32x8 tiles of
@@ -136,8 +136,7 @@ struct Slot {
     cudaArray_t tf_array[MK_MAX_LABELS] = {};
     cudaTextureObject_t tf_tex[MK_MAX_LABELS] = {};
     float *d_alpha = nullptr;           // max_labels * lut_len alpha columns
-    uint32_t *d_vis = nullptr;
-    float *d_tmax = nullptr;
+    float *d_tmax = nullptr;            // MIP bounds; for VR the bytes of the distance map and its scratch
     void *d_out = nullptr;
     void *h_stage = nullptr;            // pinned output staging
     float *h_lut = nullptr;             // pinned LUT staging (max_labels * lut_len * 4)
@@ -202,7 +201,6 @@ struct mk_server_s {
     cudaEvent_t queue_free[2] = {};
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> event_pool;
     int max_items = 0;
-    size_t vis_words = 0;
     size_t slot_bytes = 0, resident = 0, budget = 0;
 
     std::mutex mu;
@@ -255,7 +253,6 @@ void release(mk_server_s *s) {
             if (sl.tf_array[l]) cudaFreeArray(sl.tf_array[l]);
         }
         cudaFree(sl.d_alpha);
-        cudaFree(sl.d_vis);
         cudaFree(sl.d_tmax);
         cudaFree(sl.d_out);
         cudaFree(sl.d_fy);
@@ -359,9 +356,14 @@ int admit(mk_server_s *s, uint64_t ticket, int slot_index) {
             alpha_ptr[l] = l < n ? sl.d_alpha + (size_t)l * L : nullptr;
             lens[l] = l < n ? L : 0;
         }
-        int rc = launch_brick_visibility(&vs, alpha_ptr, lens, params, sl.d_vis, sl.d_tmax, s->stream);
-        if (rc != MK_OK) return rc;
-        D.bv.visible_bits = sl.d_vis;
+        const bool is_vr = q.r.kind == MK_REQUEST_VR, is_mip = q.r.kind == MK_REQUEST_MIP;
+        uint8_t *dist = reinterpret_cast<uint8_t *>(sl.d_tmax);
+        if (is_vr || is_mip) {
+            int rc = launch_brick_visibility(&vs, alpha_ptr, lens, params, is_vr ? dist : nullptr,
+                                             dist + brick_count(&vs), is_mip ? sl.d_tmax : nullptr, s->stream);
+            if (rc != MK_OK) return rc;
+        }
+        D.bv.dist = dist;
         D.bv.mip_tmax = sl.d_tmax;
         D.bv.minmax = vs.d_minmax;
         D.bv.nbx = vs.nb[0];
@@ -726,7 +728,7 @@ struct AllocInjector {
 size_t volume_estimate(int dx, int dy, int dz, bool labels) {
     const size_t nvox = (size_t)dx * dy * dz;
     const size_t nb = (size_t)((dx + 7) / 8) * ((dy + 7) / 8) * ((dz + 7) / 8);
-    return nvox * 2 + (labels ? nvox : 0) + nb * 20 + (nb / 32 + 2) * 4 + (size_t)(1.74 * dz + 16) * 4;
+    return nvox * 2 + (labels ? nvox : 0) + nb * 22 + (size_t)(1.74 * dz + 16) * 4;
 }
 
 }  // namespace
@@ -763,11 +765,9 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
     mk_server_s *s = new mk_server_s();
     s->cfg = c;
     s->budget = c.hbm_budget_bytes ? c.hbm_budget_bytes : (size_t)(0.9 * (double)free_b);
-    s->vis_words = (size_t)c.max_bricks / 32 + 2;
     s->max_items = c.tiles_per_step;
     const size_t L = (size_t)c.lut_len;
-    s->slot_bytes = (size_t)c.max_slots * ((size_t)c.max_labels * L * 20 + s->vis_words * 4 +
-                                           (size_t)c.max_bricks * 4 + (size_t)c.max_pixels * 4 + sizeof(SlotDesc)) +
+    s->slot_bytes = (size_t)c.max_slots * ((size_t)c.max_labels * L * 20 + (size_t)c.max_bricks * 4 + (size_t)c.max_pixels * 4 + sizeof(SlotDesc)) +
                     2 * (8 + (size_t)s->max_items * sizeof(TileItem));
     if (s->slot_bytes > s->budget) {
         set_last_error("mk_server_create: the slot buffers alone exceed the HBM budget");
@@ -805,7 +805,6 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
             }
             if (e != cudaSuccess) break;
             if ((e = dev_alloc((void **)&sl.d_alpha, (size_t)c.max_labels * L * sizeof(float))) != cudaSuccess) break;
-            if ((e = dev_alloc((void **)&sl.d_vis, s->vis_words * sizeof(uint32_t))) != cudaSuccess) break;
             if ((e = dev_alloc((void **)&sl.d_tmax, (size_t)c.max_bricks * sizeof(float))) != cudaSuccess) break;
             if ((e = dev_alloc((void **)&sl.d_out, (size_t)c.max_pixels * 4)) != cudaSuccess) break;
             if ((e = cudaMallocHost(&sl.h_stage, (size_t)c.max_pixels * 4)) != cudaSuccess) break;

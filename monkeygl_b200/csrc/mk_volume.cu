@@ -551,7 +551,7 @@ struct VisParams {
 __global__ void __launch_bounds__(256) k_brick_visibility(const short2 *__restrict__ minmax,
                                                           const uint32_t *__restrict__ labels,
                                                           int nbricks, VisParams P,
-                                                          uint32_t *vis_bits, float *mip_tmax) {
+                                                          uint8_t *occupied, float *mip_tmax) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     bool vis = false;
     float tmax = -INFINITY;
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(256) k_brick_visibility(const short2 *__restri
                 const float t_lo = (hu_lo - L.wl) / L.ww + 0.5f;
                 const float t_hi = (hu_hi - L.wl) / L.ww + 0.5f;
                 if (L.alpha > 0.0f) tmax = fmaxf(tmax, t_hi);
-                if (L.lut_alpha != nullptr && L.n > 0 && !vis) {
+                if (occupied && L.lut_alpha != nullptr && L.n > 0 && !vis) {
                     const float tl = fminf(t_lo, 1.0f), th = fminf(t_hi, 1.0f);
                     int i0 = (int)floorf(tl * L.n - 0.5f) - 1;
                     int i1 = (int)floorf(th * L.n - 0.5f) + 2;
@@ -593,10 +593,9 @@ __global__ void __launch_bounds__(256) k_brick_visibility(const short2 *__restri
             }
         }
         if (!(tmax == tmax)) tmax = INFINITY;
-        mip_tmax[b] = tmax;
+        if (mip_tmax) mip_tmax[b] = tmax;
+        if (occupied) occupied[b] = vis;
     }
-    const uint32_t word = __ballot_sync(0xffffffffu, vis);
-    if ((threadIdx.x & 31) == 0 && b < nbricks + 31) vis_bits[b >> 5] = word;
 }
 
 // The row kernels apply when every row splits into whole bricks and a block
@@ -659,7 +658,7 @@ float float_bound_above(double c) {
 
 BrickView brick_view(const VolumeState *v) {
     BrickView b;
-    b.visible_bits = v->d_visible;
+    b.dist = v->d_dist;
     b.mip_tmax = v->d_mip_tmax;
     b.minmax = v->d_minmax;
     b.nbx = v->nb[0];
@@ -732,7 +731,7 @@ int finish_output(VolumeState *v, void *out, size_t bytes, int out_on_device, cu
 }
 
 int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha, const int *lut_len,
-                            const float (*params)[3], uint32_t *vis_bits, float *mip_tmax, cudaStream_t s) {
+                            const float (*params)[3], uint8_t *dist, uint8_t *tmp, float *mip_tmax, cudaStream_t s) {
     const int nbricks = v->nb[0] * v->nb[1] * v->nb[2];
     VisParams P;
     for (int l = 0; l < MK_MAX_LABELS; ++l) {
@@ -744,14 +743,20 @@ int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha,
     }
     const int threads = 256;
     const int blocks = (nbricks + threads - 1) / threads;
-    k_brick_visibility<<<blocks, threads, 0, s>>>(v->d_minmax, v->d_labels, nbricks, P, vis_bits, mip_tmax);
+    k_brick_visibility<<<blocks, threads, 0, s>>>(v->d_minmax, v->d_labels, nbricks, P, dist, mip_tmax);
     MK_CUDA_TRY(cudaGetLastError());
-    return MK_OK;
+    // A run across the cube of empty bricks is up to 64 voxels long, and the
+    // schedule's rounded sums drift from the linear model by half an ulp of
+    // accuLength (< 2) a step: 64 * dim_z * 2^-24 voxels.  Up to 4096 slices
+    // that is a third of the exit margin; beyond, runs end at the brick.
+    const bool one = v->dims[2] > 4096;
+    return dist ? launch_brick_distance(dist, v->nb[0], v->nb[1], v->nb[2], one, tmp, dist, s) : MK_OK;
 }
 
 int rebuild_brick_maps(VolumeState *v, cudaStream_t s) {
     if (!v->maps_dirty) return MK_OK;
-    const int rc = launch_brick_visibility(v, v->d_tf_alpha, v->tf_len, v->params, v->d_visible, v->d_mip_tmax, s);
+    const int rc = launch_brick_visibility(v, v->d_tf_alpha, v->tf_len, v->params, v->d_dist, v->d_dist_tmp,
+                                           v->d_mip_tmax, s);
     if (rc != MK_OK) return rc;
     v->maps_dirty = false;
     return MK_OK;
@@ -840,10 +845,9 @@ extern "C" int mk_volume_create(mk_volume *out, const int16_t *voxels, int dim_x
         st.nb[1] = (dim_y + kBrick - 1) / kBrick;
         st.nb[2] = (dim_z + kBrick - 1) / kBrick;
         const size_t nbricks = (size_t)st.nb[0] * st.nb[1] * st.nb[2];
-        const size_t nwords = (nbricks + 31) / 32 + 1;
         if (cudaMalloc(&st.d_minmax, nbricks * sizeof(short2)) != cudaSuccess ||
             cudaMalloc(&st.d_labels, nbricks * 3 * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&st.d_visible, nwords * sizeof(uint32_t)) != cudaSuccess ||
+            cudaMalloc(&st.d_dist, nbricks) != cudaSuccess || cudaMalloc(&st.d_dist_tmp, nbricks) != cudaSuccess ||
             cudaMalloc(&st.d_mip_tmax, nbricks * sizeof(float)) != cudaSuccess ||
             cudaMalloc(&st.d_counter, sizeof(unsigned long long)) != cudaSuccess) {
             cudaGetLastError();
@@ -851,9 +855,8 @@ extern "C" int mk_volume_create(mk_volume *out, const int16_t *voxels, int dim_x
             rc = MK_ERR_OUT_OF_MEMORY;
             break;
         }
-        st.device_bytes += nbricks * (sizeof(short2) + 3 * sizeof(uint32_t) + sizeof(float)) +
-                           nwords * sizeof(uint32_t) + sizeof(unsigned long long);
-        cudaMemsetAsync(st.d_visible, 0, nwords * sizeof(uint32_t), st.stream);
+        st.device_bytes += nbricks * (sizeof(short2) + 3 * sizeof(uint32_t) + sizeof(float) + 2) +
+                           sizeof(unsigned long long);
         const bool staged = brick_minmax_staged_fit(dim_x, st.nb[0]);
         if (staged) {
             // d_counter doubles as the staged kernel's wait-timeout flag until the first render
@@ -935,7 +938,8 @@ extern "C" int mk_volume_destroy(mk_volume v) {
     if (st.vol_array) cudaFreeArray(st.vol_array);
     cudaFree(st.d_minmax);
     cudaFree(st.d_labels);
-    cudaFree(st.d_visible);
+    cudaFree(st.d_dist);
+    cudaFree(st.d_dist_tmp);
     cudaFree(st.d_mip_tmax);
     cudaFree(st.d_accu);
     cudaFree(st.d_out);
