@@ -52,6 +52,21 @@ __global__ void __launch_bounds__(256) k_brick_distance_z(const uint8_t *__restr
     dist[i] = (uint8_t)line_distance(in + i, nxy, (int)(i / nxy), nbz);
 }
 
+// Small grids, all three axes in one block (one launch less: 2.5 us).
+constexpr int kOneBlockBricks = 8192;
+__global__ void __launch_bounds__(1024) k_brick_distance_small(const uint8_t *occupied, int nbx, int nby, int nbz,
+                                                               uint8_t *dist) {
+    __shared__ uint8_t a[kOneBlockBricks], b[kOneBlockBricks];
+    const int nxy = nbx * nby, n = nxy * nbz;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = occupied[i] ? 0 : kMaxBrickDist;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) b[i] = (uint8_t)line_distance(a + i, 1, i % nbx, nbx);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = (uint8_t)line_distance(b + i, nbx, i / nbx % nby, nby);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) dist[i] = (uint8_t)line_distance(a + i, nxy, i / nxy, nbz);
+}
+
 // Every empty brick is its own step (also for slices too large for shared
 // memory).
 __global__ void __launch_bounds__(256) k_brick_distance_one(const uint8_t *occupied, size_t n, uint8_t *dist) {
@@ -69,6 +84,8 @@ int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, bo
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (one || 2 * nxy > kMaxSliceSmem) {
         k_brick_distance_one<<<blocks, 256, 0, s>>>(occupied, n, dist);
+    } else if (n <= kOneBlockBricks) {
+        k_brick_distance_small<<<1, 1024, 0, s>>>(occupied, nbx, nby, nbz, dist);
     } else {
         if (2 * nxy > 48 * 1024)
             MK_CUDA_TRY(cudaFuncSetAttribute(k_brick_distance_xy, cudaFuncAttributeMaxDynamicSharedMemorySize,

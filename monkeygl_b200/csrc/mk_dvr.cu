@@ -533,11 +533,13 @@ template <bool BACKWARD>
 __global__ void __launch_bounds__(256) k_dvr_build(int X, int Y, int Z, int nbx, const float *__restrict__ vol,
                                                    const float4 *__restrict__ lut, int n, float4 *__restrict__ quads,
                                                    float4 *__restrict__ gquads, uint8_t *__restrict__ needed,
-                                                   float *__restrict__ flat) {
+                                                   float *__restrict__ flat, double *__restrict__ lut_sums) {
     __shared__ float v[81][33];
     __shared__ float s_lo[8][33], s_hi[8][33];
     __shared__ int s_need[4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (BACKWARD && blockIdx.x + blockIdx.y + blockIdx.z == 0)
+        for (int i = tid; i < 4 * n; i += 256) lut_sums[i] = 0.0;
     const int x0 = blockIdx.x * 32 - 1, y0 = blockIdx.y * 8 - 1, z0 = blockIdx.z * 8 - 1;
     const int gx = min(max(x0 + lane, 0), X - 1), gx32 = min(x0 + 32, X - 1);
     float lo = INFINITY, hi = -INFINITY, lo32 = INFINITY, hi32 = -INFINITY;
@@ -623,12 +625,24 @@ __global__ void __launch_bounds__(256) k_dvr_build(int X, int Y, int Z, int nbx,
     }
 }
 
+__device__ __forceinline__ void add_lut_sums(int n, const double *__restrict__ sums, float *__restrict__ grad_lut) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        if (sums[i] != 0.0) atomicAdd(&grad_lut[i], (float)sums[i]);
+}
+
+__global__ void __launch_bounds__(256) k_dvr_lut_add(int n, const double *__restrict__ sums, float *__restrict__ grad_lut) {
+    add_lut_sums(n, sums, grad_lut);
+}
+
 // The gradient quads of one brick, summed per voxel and added to the gradient
-// volume (voxels on a brick's faces get a sum from each brick).
+// volume (voxels on a brick's faces get a sum from each brick); the first
+// block also adds the LUT sums to the LUT gradient.
 __global__ void __launch_bounds__(256) k_dvr_fold(int X, int Y, int Z, const float4 *__restrict__ gquads,
-                                                  const uint8_t *__restrict__ needed, float *__restrict__ grad_vol) {
+                                                  const uint8_t *__restrict__ needed, float *__restrict__ grad_vol,
+                                                  int n, const double *__restrict__ sums, float *__restrict__ grad_lut) {
     __shared__ float4 q[kDvrBrickQuads];
     const size_t b = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    if (b == 0) add_lut_sums(n, sums, grad_lut);
     if (needed[b] != 2) return;
     for (int i = threadIdx.x; i < kDvrBrickQuads; i += 256) q[i] = gquads[b * kDvrBrickQuads + i];
     __syncthreads();
@@ -1061,11 +1075,6 @@ k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant_
     }
 }
 
-__global__ void k_dvr_lut_add(int n, const double *__restrict__ sums, float *__restrict__ grad_lut) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && sums[i] != 0.0) atomicAdd(&grad_lut[i], (float)sums[i]);
-}
-
 // ---------------------------------------------------------------------------
 // host side
 
@@ -1172,18 +1181,25 @@ static BrickLayout brick_layout(const int dims[3], bool gradients) {
 // view of 128^2, 256^3, plain / bricks): forward 426 / 122 us where most is
 // transparent, 426 / 377 us where all is visible; backward 1256 / 734 and 1369
 // / 1312 us.  At a sixteenth the visible case turns (backward 1245 / 1401 us).
-// The exit model of a ray (linear in the sample number) holds to a few hundredths of a
+// Below about five million samples the rays must also be long (150 steps of
+// the ray parameter) for the shorter chain of a ray to outweigh three to six
+// more launches: a training step of 40^3 (depth 57) 236 / 296 us, of 90^3
+// (depth 129) 455 / 451 us, of 128^3 (depth 183) 586 / 450 us; eight 128^2
+// views of 64^3 (six million samples) 644 / 473 us.  The exit model of a ray (linear in the sample number) holds to a few hundredths of a
 // cell while a unit of the ray parameter is at most 3e4 cells along an axis;
 // quads are addressed with 32 bits.
 constexpr double kDvrSamplesPerVoxel = 0.25;
+constexpr double kDvrManySamples = 5.0e6;
+constexpr double kDvrLongRay = 150.0;
 constexpr double kDvrMaxCellsPerUnit = 3.0e4;
 
 static bool use_bricks(const mk_dvr_params *views, int nviews) {
     const mk_dvr_params &a = views[0];
-    double samples = 0.0;
+    double samples = 0.0, depth = 0.0;
     for (int i = 0; i < nviews; ++i) {
         const mk_dvr_params &p = views[i];
         samples += (double)p.width * p.height * 0.5 / p.step;
+        depth = fmax(depth, 1.0 / p.step);
         for (int k = 0; k < 3; ++k) {
             const double unit = fabs((double)p.transform[3 * k + 1] * p.scale * p.max_len_spacing[k]) * a.dims[k];
             if (!(unit <= kDvrMaxCellsPerUnit)) return false;
@@ -1193,6 +1209,7 @@ static bool use_bricks(const mk_dvr_params *views, int nviews) {
         if (a.dims[k] > 4096) return false;
     const BrickLayout l = brick_layout(a.dims, false);
     if (l.nb[1] > 65535 || l.nb[2] > 65535 || l.n * kDvrBrickQuads >= 0xffffffffull) return false;
+    if (samples < kDvrManySamples && depth < kDvrLongRay) return false;
     return samples >= kDvrSamplesPerVoxel * a.dims[0] * a.dims[1] * (double)a.dims[2];
 }
 
@@ -1209,7 +1226,7 @@ static int build_bricks(const mk_dvr_params &p, const float *volume, const float
     uint8_t *dist = reinterpret_cast<uint8_t *>(base + l.dist);
     k_dvr_build<BACKWARD><<<dim3((l.nb[0] + 3) / 4, l.nb[1], l.nb[2]), 256, 0, s>>>(
         p.dims[0], p.dims[1], p.dims[2], l.nb[0], volume, reinterpret_cast<const float4 *>(lut), p.lut_len, quads, gquads, needed,
-        flat);
+        flat, reinterpret_cast<double *>(base + l.lut));
     MK_CUDA_TRY(cudaGetLastError());
     for (int k = 0; k < 3; ++k) K.nb[k] = l.nb[k];
     K.quads = quads;
@@ -1338,7 +1355,6 @@ extern "C" int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, c
         MK_CUDA_TRY(cudaFuncSetAttribute(kern_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
         MK_CUDA_TRY(cudaFuncSetAttribute(kern_odd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         lut_sums = reinterpret_cast<double *>(static_cast<char *>(scratch) + brick_layout(views[0].dims, grad_volume != nullptr).lut);
-        MK_CUDA_TRY(cudaMemsetAsync(lut_sums, 0, 4 * views[0].lut_len * sizeof(double), s));
         rc = build_bricks<true>(views[0], volume, lut, scratch, grad_volume != nullptr, K, s);
         if (rc != MK_OK) return rc;
     } else {
@@ -1363,16 +1379,16 @@ extern "C" int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, c
         }
         MK_CUDA_TRY(cudaGetLastError());
     }
-    if (bricks) {
-        const int n = 4 * views[0].lut_len;
-        k_dvr_lut_add<<<(n + 255) / 256, 256, 0, s>>>(n, lut_sums, grad_lut);
+    if (bricks && !grad_volume) {
+        k_dvr_lut_add<<<1, 256, 0, s>>>(4 * views[0].lut_len, lut_sums, grad_lut);
         MK_CUDA_TRY(cudaGetLastError());
     }
     if (bricks && grad_volume) {
         const mk_dvr_params &p = views[0];
         const BrickLayout l = brick_layout(p.dims, true);
         k_dvr_fold<<<dim3(l.nb[0], l.nb[1], l.nb[2]), 256, 0, s>>>(
-            p.dims[0], p.dims[1], p.dims[2], K.gquads, reinterpret_cast<const uint8_t *>(scratch) + l.needed, grad_volume);
+            p.dims[0], p.dims[1], p.dims[2], K.gquads, reinterpret_cast<const uint8_t *>(scratch) + l.needed, grad_volume,
+            4 * p.lut_len, lut_sums, grad_lut);
         MK_CUDA_TRY(cudaGetLastError());
     }
     return MK_OK;
