@@ -24,6 +24,12 @@ constexpr int kBrick = 1 << kBrickShift;
 // the linear LUT filter.
 constexpr float kEmptyAlpha = 0.0004f;
 
+// Transfer-function alpha from which a sample certainly keeps a ray on step
+// L1/8: MonkeyGL's test there is 1 - (1 - alpha)^(1/8) > 0.001, alpha >
+// 0.00797; the margins absorb the rounding of the LUT filter and of powf (and
+// keep 1 - alpha positive).
+constexpr float kBusyAlpha = 0.0085f, kBusyAlphaMost = 0.999f;
+
 // Labels whose opacity cap needs a running per-ray accumulator, tracked in
 // shared memory; volumes with more such labels use the local-memory path.
 constexpr int kMaxTrackedLabels = 16;
@@ -39,6 +45,8 @@ struct LabelTable {
 struct BrickView {
     const uint8_t *dist;            // VR: 0 = some sample may have alpha > kEmptyAlpha, else the
                                     // distance to the next such brick (mk_brickdist.cu)
+    const uint8_t *busy;            // VR: l + 1 = every sample of the brick has label l and keeps a ray
+                                    // on step L1/8 (its corrected alpha is > 0.001); else 0
     const float *mip_tmax;          // MIP: upper bound of the windowed value over labels with alpha > 0
     const short2 *minmax;           // raw voxel min/max of the footprint
     int nbx, nby, nbz;
@@ -82,8 +90,9 @@ struct VolumeState {
     int nb[3] = {0, 0, 0};
     short2 *d_minmax = nullptr;
     uint32_t *d_labels = nullptr;            // 3 words (labels 0..64) per brick
-    uint8_t *d_dist = nullptr;               // VR distance map, a byte per brick, and its scratch
-    uint8_t *d_dist_tmp = nullptr;
+    uint8_t *d_dist = nullptr;               // VR distance map, a byte per brick; in the same allocation
+    uint8_t *d_dist_tmp = nullptr;           // its scratch
+    uint8_t *d_busy = nullptr;               // and the VR busy map
     float *d_mip_tmax = nullptr;
     bool maps_dirty = true;
     uint64_t present_labels[2] = {1, 0};     // labels occurring anywhere in the mask
@@ -178,12 +187,13 @@ float float_bound_above(double c);
 int ensure_device_buffer(VolumeState *v, size_t bytes);
 int ensure_pinned_buffer(VolumeState *v, size_t bytes);
 int rebuild_brick_maps(VolumeState *v, cudaStream_t s);
-// The VR distance map (dist, with scratch tmp: a byte per brick each) and MIP
-// bounds (mip_tmax) of volume v for the given per-label LUT alpha columns
+// The VR distance map (dist, with scratch tmp) and busy map (busy), a byte per
+// brick each, and the MIP bounds (mip_tmax) of volume v for the given per-label LUT alpha columns
 // (device pointers, nullptr = no table), LUT lengths and (alpha, ww, wl) rows,
-// on stream s.  Either may be null.
+// on stream s.  The three VR maps, or mip_tmax, may be null.
 int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha, const int *lut_len,
-                            const float (*params)[3], uint8_t *dist, uint8_t *tmp, float *mip_tmax, cudaStream_t s);
+                            const float (*params)[3], uint8_t *dist, uint8_t *tmp, uint8_t *busy, float *mip_tmax,
+                            cudaStream_t s);
 // Distance map over bricks (mk_brickdist.cu): `occupied` is one byte per brick
 // (0: empty), `tmp` and `dist` one byte per brick each; `dist` may be
 // `occupied`.  one: no distances, 1 for every empty brick.

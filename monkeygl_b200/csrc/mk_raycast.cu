@@ -31,6 +31,13 @@
 //    of a transfer function or window.  MIP skips bricks whose bound cannot
 //    raise the running maximum and stops at 1.0 (the 8-bit output
 //    saturates); SURFACE skips bricks whose voxels are all <= 400 HU.
+//  * Spent opacity caps.  Once a label's cap is reached its samples composite
+//    nothing, but they still hold the ray on step L1/8, eight samples a voxel
+//    and more, all through the label.  In a brick of that label alone whose
+//    transfer-function alpha is high enough everywhere to keep the step (the
+//    busy map), the ray goes to the exit in one step (labelled
+//    512x512x1559, soft tissue visible, background cap 0.4, 1024^2: 6472 ->
+//    1846 us a frame).
 //  * Warp-coherent tiles.  A 256-thread block covers a 32x8 pixel tile as
 //    eight 8x4 warp tiles, so each warp's rays are spatially adjacent and
 //    share texture cache lines; RGB output is staged in shared memory and
@@ -60,18 +67,21 @@ namespace mk {
 // (index by * tiles_x + bx): the launch takes tiles centre first, where the
 // projected volume -- and the longest rays -- usually are, so they start in
 // the first wave instead of forming the tail of the launch.  Register
-// budgets, measured on 1024^2 frames: VR 48 (five blocks per SM; four and
-// six were slower on the body and cardiac frames), MIP and surface 40 (six;
-// eight, at 32 registers, was slower).
-constexpr int kVrBlocksPerSm = 5;
+// budgets, measured on 1024^2 frames (tile launch): VR with opacity caps 64
+// registers, four blocks per SM (3 / 4 / 5: labelled 512x512x1559 142 / 145 /
+// 157 us, its dense transfer function 1920 / 1783 / 1825 us); without caps 48,
+// five (512x512x361 222 us with four, 223 with five; a 512^2 frame of
+// 128x128x96 is up to 5% slower with four, which leave it a second wave); MIP
+// and surface 40, six (eight, at 32 registers, was slower).
+constexpr int kVrBlocksPerSm = 5, kVrCappedBlocksPerSm = 4;
 constexpr int kRayBlocksPerSm = 6;
 // The hand-off launch: two blocks per SM (up to 128 registers); three and
 // four (80 and 64 registers) were slower on the body frame.
 constexpr int kTailBlocksPerSm = 2;
 template <int MODE, int TRACK, bool COUNT>
-__global__ void __launch_bounds__(256, MODE == kModeVR ? kVrBlocksPerSm : kRayBlocksPerSm) k_raycast(RayParams P, cudaTextureObject_t vol,
-                                                 cudaTextureObject_t mask, LabelTable LT,
-                                                 BrickView BV, const int *__restrict__ order) {
+__global__ void __launch_bounds__(256, MODE != kModeVR ? kRayBlocksPerSm : TRACK == kTrackNone ? kVrBlocksPerSm : kVrCappedBlocksPerSm)
+k_raycast(RayParams P, cudaTextureObject_t vol, cudaTextureObject_t mask, LabelTable LT, BrickView BV,
+          const int *__restrict__ order) {
     __shared__ LabelSmem S;
     __shared__ float s_acc[TRACK == kTrackShared ? kMaxTrackedLabels : 1][256];
     __shared__ CoopSample s_coop[MODE == kModeVR && !COUNT ? 256 : 1];
@@ -123,6 +133,7 @@ __global__ void __launch_bounds__(256, kTailBlocksPerSm) k_vr_tail(RayParams P, 
         const unsigned cnt = min(per, n - base);
         VrRay R;
         R.done = true;
+        R.cap = -1;
         R.sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if ((unsigned)lane < cnt) {
             const SpillRay &q = P.spill[base + lane];
@@ -136,6 +147,7 @@ __global__ void __launch_bounds__(256, kTailBlocksPerSm) k_vr_tail(RayParams P, 
             R.A = q.A;
             R.lat = q.lat;
             R.pix = q.pix;
+            R.cap = q.cap;
             R.done = false;
             if (TRACK == kTrackShared) {
 #pragma unroll

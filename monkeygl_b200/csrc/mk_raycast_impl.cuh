@@ -27,7 +27,8 @@ struct __align__(16) SpillRay {
     float step, aPre, A;
     int lat;
     int pix;                     // y * W + x
-    int pad[3];
+    int cap;                     // VrRay::cap
+    int pad[2];
     float acc[kMaxTrackedLabels];
 };
 
@@ -205,8 +206,7 @@ __device__ __forceinline__ StepVec step_vec(const RayParams &P) {
 // samples inside the cube is valid (they are all skippable); the margin covers
 // the rounding of the linear model.
 constexpr int kMaxRun = 240;
-__device__ __forceinline__ int steps_in_brick(const float3 &pv, const StepVec &sv, int ix, int iy, int iz,
-                                              int reach = 0) {
+__device__ __forceinline__ float time_in_brick(const float3 &pv, const StepVec &sv, int ix, int iy, int iz, int reach) {
     float t = (float)kMaxRun;
     const float e = 0.05f, back = (float)(reach * kBrick), width = (float)((2 * reach + 1) * kBrick);
     const float lo[3] = {(float)((ix >> kBrickShift) << kBrickShift) - back,
@@ -219,7 +219,12 @@ __device__ __forceinline__ int steps_in_brick(const float3 &pv, const StepVec &s
         if (rd[k] > 0.0f) t = fminf(t, (lo[k] + width - e - pp[k]) * rd[k]);
         else if (rd[k] < 0.0f) t = fminf(t, (pp[k] - lo[k] - e) * -rd[k]);
     }
-    return t > 0.0f ? (int)t : 0;
+    return fmaxf(t, 0.0f);
+}
+
+__device__ __forceinline__ int steps_in_brick(const float3 &pv, const StepVec &sv, int ix, int iy, int iz,
+                                              int reach = 0) {
+    return (int)time_in_brick(pv, sv, ix, iy, iz, reach);
 }
 
 // Advance accuLength by n coarse steps of L1.  While a ray has never refined its step it
@@ -406,6 +411,7 @@ struct VrRay {
     float4 sum;
     int lat;         // index of a in the schedule table while the step was never refined, else -1
     int pix;         // y * W + x of the ray's pixel
+    int cap;         // label of the last sample if its opacity cap kept it out on step L1/8, else -1
     bool done;
 };
 
@@ -442,6 +448,7 @@ __device__ __forceinline__ bool spill_ray(const RayParams &P, const VrRay &R, co
     o.A = R.A;
     o.lat = R.lat;
     o.pix = R.pix;
+    o.cap = R.cap;
     if (TRACK == kTrackShared) {
 #pragma unroll
         for (int k = 0; k < kMaxTrackedLabels; ++k) o.acc[k] = s_acc[k][acc_tid];
@@ -509,6 +516,7 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
             T.sum.w = __shfl_sync(FULL, Q.sum.w, src);
             T.lat = __shfl_sync(FULL, Q.lat, src);
             T.pix = __shfl_sync(FULL, Q.pix, src);
+            T.cap = TRACK != kTrackNone ? __shfl_sync(FULL, Q.cap, src) : -1;
             // masked to a lane: a shuffled value indexes the warp's own
             // slices of s_acc and ws, so even a value from a lane that did
             // not take part cannot address outside them
@@ -527,6 +535,16 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
             // 1..hA the refined run, lanes hA+1.. the coarsened run; the
             // sample's test picks the run that is walked.
             const bool two = G >= 8 && !Q.done && Q.step == L4 && Q.a > 0.0f;
+            // opacity cap spent: across the busy bricks of the label first (vr_march)
+            while (TRACK != kTrackNone && P.skip && Q.cap >= 0 && !Q.done && Q.a < P.limit && !(Q.a > Q.a_stop)) {
+                const float3 pos = ray_pos(P, Q.u, Q.v, Q.a);
+                const int ix = pos.x * P.fdim[0];
+                const int iy = pos.y * P.fdim[1];
+                const int iz = pos.z * P.fdim[2];
+                if (outside_voi(P, ix, iy, iz) || BV.busy[brick_index(P, BV, ix, iy, iz)] != Q.cap + 1) break;
+                const float3 pv = make_float3(pos.x * P.fdim[0], pos.y * P.fdim[1], pos.z * P.fdim[2]);
+                Q.a = add_steps(Q.a, Q.step, 1 + (int)(8.0f * time_in_brick(pv, dv, ix, iy, iz, 0)));
+            }
             const int hA = G / 2 - 1;
             // 1. this lane's sample: j steps ahead, or its place in its run
             float4 clr = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -687,6 +705,7 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
                     int c_lab = -1, c_slot = -2;
                     float c_cap = 0.0f, c_acc = 0.0f;
                     bool ended = false;
+                    int last_out = -1;       // VrRay::cap after the round
                     int k = lead0 ? 0 : r_lo;
                     float alpha_n = gs[k].alpha;
                     int meta_n = gs[k].meta;
@@ -702,6 +721,7 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
                             clr_n = gs[kn].clr;
                         }
                         k = kn;
+                        last_out = -1;
                         if (alpha > 0.0005f) {
                             if (lab != c_lab) {
                                 if (TRACK == kTrackShared && c_slot >= 0) s_acc[c_slot][owner_tid] = c_acc;
@@ -711,6 +731,7 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
                                 c_acc = (TRACK == kTrackShared && c_slot >= 0) ? s_acc[c_slot][owner_tid] : 0.0f;
                             }
                             const bool ok = c_slot != -2 && (c_slot == -1 || TRACK != kTrackShared || c_acc < c_cap);
+                            if (!ok && step_new == L8 && alpha > 0.001f && a_new > L8) last_out = lab;
                             if (ok) {
                                 Q.sum = composite(Q.sum, Q.A, alpha, clr);
                                 if (TRACK == kTrackShared && c_slot >= 0) c_acc += (1.0f - Q.A) * alpha;
@@ -730,10 +751,12 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
                         Q.aPre = pre_new;
                         Q.step = step_new;
                         Q.lat = lat_new;
+                        Q.cap = last_out;
                     }
                 }
             }
             if (!simple && !Q.done) {
+                Q.cap = -1;
                 // The walk is the serial part of a round, so nothing on its
                 // chain waits for shared memory: the next sample is read
                 // while this one is walked, and the opacity cap of the label
@@ -890,6 +913,7 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
     R.sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     R.lat = -1;
     R.pix = y * P.W + x;
+    R.cap = -1;
     R.done = true;
     if (active) {
         R.u = 1.0f * (x - P.W / 2.0f - P.xT) / P.H;
@@ -951,6 +975,16 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
                     if (R.lat >= 0) ++R.lat;
                     break;
                 }
+                if (TRACK != kTrackNone && P.skip && R.cap >= 0) {
+                    // Opacity cap spent, step L1/8: in a brick of this label
+                    // whose samples all keep the step, nothing happens before
+                    // its exit.  (Of aPre only aPre > 0.001 matters.)
+                    if (BV.busy[brick_index(P, BV, ix, iy, iz)] == R.cap + 1) {
+                        const float3 pv = make_float3(pos.x * P.fdim[0], pos.y * P.fdim[1], pos.z * P.fdim[2]);
+                        R.a = add_steps(R.a, R.step, 1 + (int)(8.0f * time_in_brick(pv, dv, ix, iy, iz, 0)));
+                        break;
+                    }
+                }
                 if (P.skip && R.step == L1 && R.aPre <= 0.001f) {
                     const int dist = BV.dist[brick_index(P, BV, ix, iy, iz)];
                     if (dist != 0) {
@@ -991,7 +1025,10 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
                 R.a += R.step;
                 if (R.lat >= 0) ++R.lat;
                 col.w = alpha;
-                if (col.w > 0.0005f && vr_cap_ok<TRACK>(S, s_acc, accLocal, label, tid)) {
+                if (TRACK != kTrackNone) R.cap = -1;
+                if (col.w > 0.0005f && !vr_cap_ok<TRACK>(S, s_acc, accLocal, label, tid)) {
+                    if (TRACK != kTrackNone && R.step == L8 && R.a > L8 && alpha > 0.001f) R.cap = label;
+                } else if (col.w > 0.0005f) {
                     R.sum = composite(R.sum, R.A, col.w, shade_color(vol, pos, col, L, P));
                     vr_cap_add<TRACK>(S, s_acc, accLocal, label, tid, R.A, col.w);
                     R.A += (1.0f - R.A) * col.w;

@@ -136,7 +136,7 @@ struct Slot {
     cudaArray_t tf_array[MK_MAX_LABELS] = {};
     cudaTextureObject_t tf_tex[MK_MAX_LABELS] = {};
     float *d_alpha = nullptr;           // max_labels * lut_len alpha columns
-    float *d_tmax = nullptr;            // MIP bounds; for VR the bytes of the distance map and its scratch
+    float *d_tmax = nullptr;            // MIP bounds; for VR the bytes of the distance map, its scratch and the busy map
     void *d_out = nullptr;
     void *h_stage = nullptr;            // pinned output staging
     float *h_lut = nullptr;             // pinned LUT staging (max_labels * lut_len * 4)
@@ -359,11 +359,13 @@ int admit(mk_server_s *s, uint64_t ticket, int slot_index) {
         const bool is_vr = q.r.kind == MK_REQUEST_VR, is_mip = q.r.kind == MK_REQUEST_MIP;
         uint8_t *dist = reinterpret_cast<uint8_t *>(sl.d_tmax);
         if (is_vr || is_mip) {
-            int rc = launch_brick_visibility(&vs, alpha_ptr, lens, params, is_vr ? dist : nullptr,
-                                             dist + brick_count(&vs), is_mip ? sl.d_tmax : nullptr, s->stream);
+            const size_t nb = brick_count(&vs);
+            int rc = launch_brick_visibility(&vs, alpha_ptr, lens, params, is_vr ? dist : nullptr, dist + nb,
+                                             is_vr ? dist + 2 * nb : nullptr, is_mip ? sl.d_tmax : nullptr, s->stream);
             if (rc != MK_OK) return rc;
         }
         D.bv.dist = dist;
+        D.bv.busy = dist + 2 * brick_count(&vs);
         D.bv.mip_tmax = sl.d_tmax;
         D.bv.minmax = vs.d_minmax;
         D.bv.nbx = vs.nb[0];
@@ -728,7 +730,7 @@ struct AllocInjector {
 size_t volume_estimate(int dx, int dy, int dz, bool labels) {
     const size_t nvox = (size_t)dx * dy * dz;
     const size_t nb = (size_t)((dx + 7) / 8) * ((dy + 7) / 8) * ((dz + 7) / 8);
-    return nvox * 2 + (labels ? nvox : 0) + nb * 22 + (size_t)(1.74 * dz + 16) * 4;
+    return nvox * 2 + (labels ? nvox : 0) + nb * 23 + (size_t)(1.74 * dz + 16) * 4;
 }
 
 }  // namespace

@@ -551,11 +551,12 @@ struct VisParams {
 __global__ void __launch_bounds__(256) k_brick_visibility(const short2 *__restrict__ minmax,
                                                           const uint32_t *__restrict__ labels,
                                                           int nbricks, VisParams P,
-                                                          uint8_t *occupied, float *mip_tmax) {
+                                                          uint8_t *occupied, uint8_t *busy, float *mip_tmax) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     bool vis = false;
     float tmax = -INFINITY;
     if (b < nbricks) {
+        int only = -1, n_labels = 0;         // the brick's label, if it has one only
         const short2 mm = minmax[b];
         // Normalized-float read of int16 is v/32767; the kernels scale it by
         // 32768 (core/kernel.cu:223).  Widen for the filter's rounding.
@@ -572,6 +573,8 @@ __global__ void __launch_bounds__(256) k_brick_visibility(const short2 *__restri
                 const VisLabel L = P.lab[l];
                 const float t_lo = (hu_lo - L.wl) / L.ww + 0.5f;
                 const float t_hi = (hu_hi - L.wl) / L.ww + 0.5f;
+                only = l;
+                ++n_labels;
                 if (L.alpha > 0.0f) tmax = fmaxf(tmax, t_hi);
                 if (occupied && L.lut_alpha != nullptr && L.n > 0 && !vis) {
                     const float tl = fminf(t_lo, 1.0f), th = fminf(t_hi, 1.0f);
@@ -593,6 +596,21 @@ __global__ void __launch_bounds__(256) k_brick_visibility(const short2 *__restri
             }
         }
         if (!(tmax == tmax)) tmax = INFINITY;
+        if (busy) {
+            bool all = false;
+            if (vis && n_labels == 1) {
+                const VisLabel L = P.lab[only];
+                const float t_lo = (hu_lo - L.wl) / L.ww + 0.5f, t_hi = (hu_hi - L.wl) / L.ww + 0.5f;
+                if (t_lo == t_lo && t_hi == t_hi) {
+                    const int i0 = max(0, min((int)floorf(fminf(t_lo, 1.0f) * L.n - 0.5f) - 1, L.n - 1));
+                    const int i1 = max(0, min((int)floorf(fminf(t_hi, 1.0f) * L.n - 0.5f) + 2, L.n - 1));
+                    all = true;
+                    for (int i = i0; i <= i1 && all; ++i)
+                        all = L.lut_alpha[i] >= kBusyAlpha && L.lut_alpha[i] <= kBusyAlphaMost;
+                }
+            }
+            busy[b] = all ? (uint8_t)(only + 1) : 0;
+        }
         if (mip_tmax) mip_tmax[b] = tmax;
         if (occupied) occupied[b] = vis;
     }
@@ -659,6 +677,7 @@ float float_bound_above(double c) {
 BrickView brick_view(const VolumeState *v) {
     BrickView b;
     b.dist = v->d_dist;
+    b.busy = v->d_busy;
     b.mip_tmax = v->d_mip_tmax;
     b.minmax = v->d_minmax;
     b.nbx = v->nb[0];
@@ -731,7 +750,8 @@ int finish_output(VolumeState *v, void *out, size_t bytes, int out_on_device, cu
 }
 
 int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha, const int *lut_len,
-                            const float (*params)[3], uint8_t *dist, uint8_t *tmp, float *mip_tmax, cudaStream_t s) {
+                            const float (*params)[3], uint8_t *dist, uint8_t *tmp, uint8_t *busy, float *mip_tmax,
+                            cudaStream_t s) {
     const int nbricks = v->nb[0] * v->nb[1] * v->nb[2];
     VisParams P;
     for (int l = 0; l < MK_MAX_LABELS; ++l) {
@@ -741,22 +761,27 @@ int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha,
         P.lab[l].ww = params[l][1];
         P.lab[l].wl = params[l][2];
     }
-    const int threads = 256;
-    const int blocks = (nbricks + threads - 1) / threads;
-    k_brick_visibility<<<blocks, threads, 0, s>>>(v->d_minmax, v->d_labels, nbricks, P, dist, mip_tmax);
-    MK_CUDA_TRY(cudaGetLastError());
     // A run across the cube of empty bricks is up to 64 voxels long, and the
     // schedule's rounded sums drift from the linear model by half an ulp of
     // accuLength (< 2) a step: 64 * dim_z * 2^-24 voxels.  Up to 4096 slices
-    // that is a third of the exit margin; beyond, runs end at the brick.
+    // that is a third of the exit margin; beyond, runs end at the brick and
+    // there are none on step L1/8 (which takes as many steps across a brick).
     const bool one = v->dims[2] > 4096;
+    if (one && busy) {
+        MK_CUDA_TRY(cudaMemsetAsync(busy, 0, (size_t)nbricks, s));
+        busy = nullptr;
+    }
+    const int threads = 256;
+    const int blocks = (nbricks + threads - 1) / threads;
+    k_brick_visibility<<<blocks, threads, 0, s>>>(v->d_minmax, v->d_labels, nbricks, P, dist, busy, mip_tmax);
+    MK_CUDA_TRY(cudaGetLastError());
     return dist ? launch_brick_distance(dist, v->nb[0], v->nb[1], v->nb[2], one, tmp, dist, s) : MK_OK;
 }
 
 int rebuild_brick_maps(VolumeState *v, cudaStream_t s) {
     if (!v->maps_dirty) return MK_OK;
     const int rc = launch_brick_visibility(v, v->d_tf_alpha, v->tf_len, v->params, v->d_dist, v->d_dist_tmp,
-                                           v->d_mip_tmax, s);
+                                           v->d_busy, v->d_mip_tmax, s);
     if (rc != MK_OK) return rc;
     v->maps_dirty = false;
     return MK_OK;
@@ -847,7 +872,7 @@ extern "C" int mk_volume_create(mk_volume *out, const int16_t *voxels, int dim_x
         const size_t nbricks = (size_t)st.nb[0] * st.nb[1] * st.nb[2];
         if (cudaMalloc(&st.d_minmax, nbricks * sizeof(short2)) != cudaSuccess ||
             cudaMalloc(&st.d_labels, nbricks * 3 * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&st.d_dist, nbricks) != cudaSuccess || cudaMalloc(&st.d_dist_tmp, nbricks) != cudaSuccess ||
+            cudaMalloc(&st.d_dist, 3 * nbricks) != cudaSuccess ||
             cudaMalloc(&st.d_mip_tmax, nbricks * sizeof(float)) != cudaSuccess ||
             cudaMalloc(&st.d_counter, sizeof(unsigned long long)) != cudaSuccess) {
             cudaGetLastError();
@@ -855,7 +880,9 @@ extern "C" int mk_volume_create(mk_volume *out, const int16_t *voxels, int dim_x
             rc = MK_ERR_OUT_OF_MEMORY;
             break;
         }
-        st.device_bytes += nbricks * (sizeof(short2) + 3 * sizeof(uint32_t) + sizeof(float) + 2) +
+        st.d_dist_tmp = st.d_dist + nbricks;
+        st.d_busy = st.d_dist + 2 * nbricks;
+        st.device_bytes += nbricks * (sizeof(short2) + 3 * sizeof(uint32_t) + sizeof(float) + 3) +
                            sizeof(unsigned long long);
         const bool staged = brick_minmax_staged_fit(dim_x, st.nb[0]);
         if (staged) {
@@ -939,7 +966,7 @@ extern "C" int mk_volume_destroy(mk_volume v) {
     cudaFree(st.d_minmax);
     cudaFree(st.d_labels);
     cudaFree(st.d_dist);
-    cudaFree(st.d_dist_tmp);
+
     cudaFree(st.d_mip_tmax);
     cudaFree(st.d_accu);
     cudaFree(st.d_out);
