@@ -182,6 +182,8 @@ void set_last_error(const std::string &msg);
 // Smallest float strictly greater than the double bound c; for a float a,
 // a < c  <=>  a < float_bound_above(c) when c is not itself a float.
 float float_bound_above(double c);
+// Smallest float >= c; for a float a, a < c  <=>  a < float_bound_at(c).
+float float_bound_at(double c);
 
 // Host helpers shared by the entry points.
 int ensure_device_buffer(VolumeState *v, size_t bytes);

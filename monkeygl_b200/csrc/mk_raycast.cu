@@ -67,19 +67,18 @@ namespace mk {
 // (index by * tiles_x + bx): the launch takes tiles centre first, where the
 // projected volume -- and the longest rays -- usually are, so they start in
 // the first wave instead of forming the tail of the launch.  Register
-// budgets, measured on 1024^2 frames (tile launch): VR with opacity caps 64
-// registers, four blocks per SM (3 / 4 / 5: labelled 512x512x1559 142 / 145 /
-// 157 us, its dense transfer function 1920 / 1783 / 1825 us); without caps 48,
-// five (512x512x361 222 us with four, 223 with five; a 512^2 frame of
-// 128x128x96 is up to 5% slower with four, which leave it a second wave); MIP
-// and surface 40, six (eight, at 32 registers, was slower).
-constexpr int kVrBlocksPerSm = 5, kVrCappedBlocksPerSm = 4;
+// budgets, measured on tile launches: VR 64 registers, four blocks per SM
+// (against five, which spill: 512^2 of 128x128x96 139 / 147 us, 1024^2 of
+// 512x512x361 178 / 190 us, labelled 512x512x1559 140 / 157 us; three: the
+// latter's dense transfer function 1783 -> 1920 us); MIP and surface 40, six
+// (MIP 1024^2 of 512x512x361 with five / six / eight: 323 / 316 / 341 us).
+constexpr int kVrBlocksPerSm = 4;
 constexpr int kRayBlocksPerSm = 6;
 // The hand-off launch: two blocks per SM (up to 128 registers); three and
 // four (80 and 64 registers) were slower on the body frame.
 constexpr int kTailBlocksPerSm = 2;
 template <int MODE, int TRACK, bool COUNT>
-__global__ void __launch_bounds__(256, MODE != kModeVR ? kRayBlocksPerSm : TRACK == kTrackNone ? kVrBlocksPerSm : kVrCappedBlocksPerSm)
+__global__ void __launch_bounds__(256, MODE == kModeVR ? kVrBlocksPerSm : kRayBlocksPerSm)
 k_raycast(RayParams P, cudaTextureObject_t vol, cudaTextureObject_t mask, LabelTable LT, BrickView BV,
           const int *__restrict__ order) {
     __shared__ LabelSmem S;
@@ -561,6 +560,13 @@ int fill_ray_params(const VolumeState &v, const mk_vr_params *p, RayParams &P) {
     for (int i = 0; i < 9; ++i) P.M[i] = p->transform[i];
     P.invertZ = p->invert_z ? 1 : 0;
     for (int i = 0; i < 6; ++i) P.voi[i] = p->voi[i];
+    // trunc(x) >= v: x >= v for v > 0, else x > v - 1; trunc(x) <= v: x < v + 1
+    // for v >= 0, else x <= v
+    for (int k = 0; k < 3; ++k) {
+        const double lo = p->voi[2 * k], hi = p->voi[2 * k + 1];
+        P.voi_lo[k] = lo > 0 ? float_bound_at(lo) : float_bound_above(lo - 1);
+        P.voi_hi[k] = hi >= 0 ? float_bound_at(hi + 1) : float_bound_above(hi);
+    }
     P.bg = make_float4(p->background[0], p->background[1], p->background[2], p->background[3]);
     P.step1 = 1.0f / (float)v.dims[2];
     P.limit = float_bound_above(1.732);
@@ -579,6 +585,14 @@ int fill_ray_params(const VolumeState &v, const mk_vr_params *p, RayParams &P) {
     P.spill_cap = 0;
     P.tail_trigger = 0;
     P.patch = nullptr;
+    // the rounding of a position, in voxels: the terms of its camera product
+    // are up to this large
+    P.interior = 1;
+    const double um = (0.5 * P.W + fabs((double)P.xT)) / P.H, vm = (0.5 * P.H + fabs((double)P.yT)) / P.H;
+    for (int k = 0; k < 3; ++k) {
+        const double t = um * fabs((double)P.M[3 * k]) + 0.87 * P.scale * fabs((double)P.M[3 * k + 1]) + vm * fabs((double)P.M[3 * k + 2]);
+        if (!((t * fabs((double)P.mls[k]) + 1.0) * P.fdim[k] * 4.8e-7 < 0.1)) P.interior = 0;
+    }
     P.mip_uniform = 0;
     P.mip_ww = 1.0f;
     P.mip_wl = 0.0f;

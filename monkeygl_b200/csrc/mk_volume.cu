@@ -674,6 +674,12 @@ float float_bound_above(double c) {
     return f;
 }
 
+float float_bound_at(double c) {
+    float f = (float)c;
+    if ((double)f < c) f = nextafterf(f, INFINITY);
+    return f;
+}
+
 BrickView brick_view(const VolumeState *v) {
     BrickView b;
     b.dist = v->d_dist;
