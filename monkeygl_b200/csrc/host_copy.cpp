@@ -1,0 +1,140 @@
+// host_copy.cpp -- finished images from pinned staging memory to the caller's
+// pageable buffer by several threads.
+//
+// The bytes come fresh from the device's DMA, so one thread's memcpy runs at
+// memory latency (measured 24 us for 512 KB, 47 us for 1 MB, 200 us for 3 MB,
+// against 10 / 19 / 55 us for the DMA itself).  Up to three helper threads,
+// kept by the process and asleep between images, are woken while the GPU still
+// works and then share the copy in 64 KB pieces with the calling thread.  The
+// caller takes pieces too and needs no helper to finish: one that wakes late,
+// or no longer exists (a forked child), finds or leaves nothing to do.  One
+// caller at a time has the helpers; another copies alone.
+#include <string.h>
+
+#include <algorithm>
+#include <atomic>
+#include <chrono>
+#include <condition_variable>
+#include <mutex>
+#include <new>
+#include <system_error>
+#include <thread>
+
+#include "mk_internal.h"
+
+namespace mk {
+
+namespace {
+
+constexpr size_t kPiece = 64u << 10;
+constexpr size_t kHelpMin = 256u << 10;     // smaller images: the caller alone
+constexpr int kHelpers = 3;
+constexpr auto kSpin = std::chrono::microseconds(200);
+
+inline void pause_cpu() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#else
+    std::this_thread::yield();
+#endif
+}
+
+struct CopyPool {
+    std::mutex owner;                        // held by the caller that has the helpers
+    std::mutex mu;
+    std::condition_variable cv;
+    uint64_t wakes = 0;                      // guarded by mu
+    // generation of the copy (high 32 bits) and its next piece; a piece is
+    // taken by advancing it under the same generation
+    std::atomic<uint64_t> ticket{0};
+    std::atomic<uint32_t> done{0};
+    char *dst = nullptr;
+    const char *src = nullptr;
+    size_t bytes = 0;
+    std::atomic<uint32_t> pieces{0};
+
+    bool take(uint32_t gen) {
+        uint64_t t = ticket.load(std::memory_order_acquire);
+        for (;;) {
+            if ((uint32_t)(t >> 32) != gen || (uint32_t)t >= pieces.load(std::memory_order_relaxed)) return false;
+            if (ticket.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel, std::memory_order_acquire)) break;
+        }
+        // the piece is this thread's, and the copy cannot end without it
+        const size_t off = (size_t)(uint32_t)t * kPiece;
+        memcpy(dst + off, src + off, std::min(kPiece, bytes - off));
+        done.fetch_add(1, std::memory_order_release);
+        return true;
+    }
+
+    void helper() {
+        uint64_t seen = 0;
+        uint32_t gen = 0;
+        for (;;) {
+            {
+                std::unique_lock<std::mutex> lk(mu);
+                cv.wait(lk, [&] { return wakes != seen; });
+                seen = wakes;
+            }
+            const auto until = std::chrono::steady_clock::now() + kSpin;
+            for (int i = 0;; ++i) {
+                const uint32_t g = (uint32_t)(ticket.load(std::memory_order_acquire) >> 32);
+                if (g != gen) {
+                    gen = g;
+                    while (take(g)) {
+                    }
+                    break;
+                }
+                if ((i & 63) == 63 && std::chrono::steady_clock::now() > until) break;
+                pause_cpu();
+            }
+        }
+    }
+
+    CopyPool() {
+        if (std::thread::hardware_concurrency() < 2 * (kHelpers + 1)) return;
+        try {
+            for (int i = 0; i < kHelpers; ++i) std::thread([this] { helper(); }).detach();
+        } catch (const std::system_error &) {    // fewer helpers, or none
+        }
+    }
+};
+
+CopyPool *pool() {
+    static CopyPool *p = new (std::nothrow) CopyPool();   // kept until the process exits, like its threads
+    return p;
+}
+
+}  // namespace
+
+void copy_out_soon(size_t bytes) {
+    if (bytes < kHelpMin) return;
+    CopyPool *p = pool();
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(p->mu);
+        ++p->wakes;
+    }
+    p->cv.notify_all();
+}
+
+void copy_out(void *dst, const void *src, size_t bytes) {
+    CopyPool *p = bytes < kHelpMin ? nullptr : pool();
+    if (!p || !p->owner.try_lock()) {
+        memcpy(dst, src, bytes);
+        return;
+    }
+    const uint32_t n = (uint32_t)((bytes + kPiece - 1) / kPiece);
+    const uint32_t gen = (uint32_t)(p->ticket.load(std::memory_order_relaxed) >> 32) + 1;
+    p->dst = static_cast<char *>(dst);
+    p->src = static_cast<const char *>(src);
+    p->bytes = bytes;
+    p->done.store(0, std::memory_order_relaxed);
+    p->pieces.store(n, std::memory_order_relaxed);
+    p->ticket.store((uint64_t)gen << 32, std::memory_order_release);
+    while (p->take(gen)) {
+    }
+    while (p->done.load(std::memory_order_acquire) != n) pause_cpu();
+    p->owner.unlock();
+}
+
+}  // namespace mk

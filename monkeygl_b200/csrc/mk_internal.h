@@ -205,6 +205,10 @@ int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, bo
 // Bytes of the distance map / floats of MIP bounds of a volume's brick maps.
 inline size_t brick_count(const VolumeState *v) { return (size_t)v->nb[0] * v->nb[1] * v->nb[2]; }
 int finish_output(VolumeState *v, void *out, size_t bytes, int out_on_device, cudaStream_t s);
+// Copy of a finished image out of pinned staging memory (host_copy.cpp);
+// copy_out_soon wakes the helper threads while the GPU still works on it.
+void copy_out_soon(size_t bytes);
+void copy_out(void *dst, const void *src, size_t bytes);
 // True for page-locked host memory the device can copy to directly.
 bool is_pinned_host(const void *p);
 BrickView brick_view(const VolumeState *v);

@@ -668,9 +668,15 @@ extern "C" int mk_render_vr(mk_volume vol, const mk_vr_params *params, void *out
     if (rc == MK_OK) rc = note_table_use(v.fy_tables[fy_idx].uses, s);
     if (rc != MK_OK) return rc;
     if (!tb) return finish_output(&v, out, bytes, out_on_device, s);
+    // (the image is usually here before the hand-off launch ends, so it goes
+    // to the caller's buffer meanwhile)
+    if (dst != out) {
+        MK_CUDA_TRY(cudaEventSynchronize(tb->tiles_done));
+        copy_out_soon(bytes);
+    }
     MK_CUDA_TRY(cudaStreamSynchronize(tb->copy_stream));
+    if (dst != out) copy_out(out, dst, bytes);
     MK_CUDA_TRY(cudaStreamSynchronize(s));
-    if (dst != out) memcpy(out, dst, bytes);
     // the tail launch's pixels, from its (pix, rgb) list in mapped memory
     const volatile uint32_t *pl = tb->h_patch;
     const uint32_t n_listed = pl[0];

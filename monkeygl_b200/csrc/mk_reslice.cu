@@ -224,13 +224,6 @@ extern "C" int mk_render_cpr(mk_volume vol, int width, int height, const double 
     VolumeState &v = vol->st;
     cudaSetDevice(v.device);
     cudaStream_t s = stream ? (cudaStream_t)stream : v.stream;
-    std::vector<CprRow> rows(height);
-    for (int y = 0; y < height; ++y) {
-        for (int k = 0; k < 3; ++k) {
-            rows[y].p[k] = points[3 * y + k];
-            rows[y].d[k] = dirs[3 * y + k];
-        }
-    }
     const size_t out_bytes = (size_t)width * height * sizeof(short);
     const size_t row_bytes = (size_t)height * sizeof(CprRow);
     const size_t row_off = (out_bytes + 255) & ~(size_t)255;
@@ -239,7 +232,13 @@ extern "C" int mk_render_cpr(mk_volume vol, int width, int height, const double 
     CprRow *d_rows = reinterpret_cast<CprRow *>(static_cast<char *>(v.d_out) + row_off);
     rc = ensure_pinned_buffer(&v, row_bytes);
     if (rc != MK_OK) return rc;
-    memcpy(v.h_pinned, rows.data(), row_bytes);
+    CprRow *rows = static_cast<CprRow *>(v.h_pinned);
+    for (int y = 0; y < height; ++y) {
+        for (int k = 0; k < 3; ++k) {
+            rows[y].p[k] = points[3 * y + k];
+            rows[y].d[k] = dirs[3 * y + k];
+        }
+    }
     MK_CUDA_TRY(cudaMemcpyAsync(d_rows, v.h_pinned, row_bytes, cudaMemcpyHostToDevice, s));
     short *dst = out_on_device ? out : static_cast<short *>(v.d_out);
     dim3 grid((width + 31) / 32, (height + 7) / 8);

@@ -750,8 +750,9 @@ int finish_output(VolumeState *v, void *out, size_t bytes, int out_on_device, cu
     int st = ensure_pinned_buffer(v, bytes);
     if (st != MK_OK) return st;
     MK_CUDA_TRY(cudaMemcpyAsync(v->h_pinned, v->d_out, bytes, cudaMemcpyDeviceToHost, s));
+    copy_out_soon(bytes);
     MK_CUDA_TRY(cudaStreamSynchronize(s));
-    memcpy(out, v->h_pinned, bytes);
+    copy_out(out, v->h_pinned, bytes);
     return MK_OK;
 }
 
