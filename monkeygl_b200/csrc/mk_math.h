@@ -70,4 +70,35 @@ MK_HD float add_steps(float a, float step, int n) {
     return a;
 }
 
+// Pixel of thread t in a 32x8 tile of a 256-thread block: eight 8x4 warp tiles,
+// and inside one the lanes along a Z curve, so that the four lanes the texture
+// unit serves together are 2x2 pixels and touch fewer texels than four in a
+// row.
+MK_HD int tile_x(int t) { return ((t >> 5) & 3) * 8 + ((t & 1) | ((t >> 1) & 2) | ((t >> 2) & 4)); }
+MK_HD int tile_y(int t) { return (t >> 7) * 4 + (((t >> 1) & 1) | ((t >> 2) & 2)); }
+
+// a / d, correctly rounded, given y = 1 / d correctly rounded: two corrections
+// of a * y by the remainder, which one fused multiply-add gives (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34(1), 1990: with y correctly rounded, the correction of a
+// quotient within one ulp is correctly rounded; the first correction brings a * y
+// there).  For d, 1 / d and a / d well inside the range of normal numbers
+// (div_by_ok); an infinite a gives NaN.
+MK_HD float div_by(float a, float d, float y) {
+    float q = a * y;
+    q = fmaf(fmaf(-q, d, a), y, q);
+    return fmaf(fmaf(-q, d, a), y, q);
+}
+
+MK_HD double div_by(double a, double d, double y) {
+    double q = a * y;
+    q = fma(fma(-q, d, a), y, q);
+    return fma(fma(-q, d, a), y, q);
+}
+
+MK_HD bool div_by_ok(float d) {
+    const float m = fabsf(d);
+    return m >= 1e-18f && m <= 1e18f;
+}
+
 }  // namespace mk

@@ -12,9 +12,9 @@
 // operation (FP64 runs at half the FP32 rate on sm_100).  MK_SAMPLE_NEAREST reads the same voxels through a
 // point-filtered texture view.
 //
-// Layout: 256-thread blocks cover 32x8 output tiles so each warp stores one
-// 64-byte row segment; CPR rows share their (point, direction) pair through
-// shared memory.
+// Layout: 256-thread blocks cover 32x8 output tiles as 8x4 warp tiles, four
+// lanes to 2x2 pixels (tile_x in mk_math.h); CPR rows share their (point,
+// direction) pair through shared memory.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -41,25 +41,40 @@ struct CprRow {
 
 // (float)((p + x * dir) / n) in double, operation for operation as nvcc
 // compiles core/kernel.cu:860-862 (the multiply-add fused; the CPR parity
-// tests compare every pixel with MonkeyGL's kernel).
-__device__ __forceinline__ float cpr_coord_d(double p, double d, int x, float n) {
-    return __double2float_rn(__ddiv_rn(__fma_rn((double)x, d, p), (double)n));
+// tests compare every pixel with MonkeyGL's kernel), the quotient by div_by
+// with inv = 1 / n (n is a dimension; beyond 1e300 by division).
+__device__ __forceinline__ float cpr_coord_d(double p, double d, int x, double n, double inv) {
+    const double a = __fma_rn((double)x, d, p);
+    return __double2float_rn(fabs(a) < 1e300 ? div_by(a, n, inv) : __ddiv_rn(a, n));
 }
 
-__global__ void __launch_bounds__(256) k_cpr(int W, int H, float3 fdim, int invertZ,
+// Dimensions of the volume and their reciprocals.
+struct CprDims {
+    double n[3], inv[3];
+};
+
+static CprDims cpr_dims(const VolumeState &v) {
+    CprDims c;
+    for (int k = 0; k < 3; ++k) {
+        c.n[k] = (double)(float)v.dims[k];
+        c.inv[k] = 1.0 / c.n[k];
+    }
+    return c;
+}
+
+__global__ void __launch_bounds__(256) k_cpr(int W, int H, const __grid_constant__ CprDims dim, int invertZ,
                                              const CprRow *__restrict__ rows,
                                              cudaTextureObject_t tex, short *out) {
     __shared__ CprRow s_rows[8];
-    const int ly = threadIdx.x >> 5;
-    const int y = blockIdx.y * 8 + ly;
-    if ((threadIdx.x & 31) == 0 && y < H) s_rows[ly] = rows[y];
+    if (threadIdx.x < 8 && blockIdx.y * 8 + threadIdx.x < H) s_rows[threadIdx.x] = rows[blockIdx.y * 8 + threadIdx.x];
     __syncthreads();
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+    const int ly = tile_y(threadIdx.x);
+    const int x = blockIdx.x * 32 + tile_x(threadIdx.x), y = blockIdx.y * 8 + ly;
     if (x >= W || y >= H) return;
     const CprRow &R = s_rows[ly];
-    const float fx = cpr_coord_d(R.p[0], R.d[0], x, fdim.x);
-    const float fy = cpr_coord_d(R.p[1], R.d[1], x, fdim.y);
-    float fz = cpr_coord_d(R.p[2], R.d[2], x, fdim.z);
+    const float fx = cpr_coord_d(R.p[0], R.d[0], x, dim.n[0], dim.inv[0]);
+    const float fy = cpr_coord_d(R.p[1], R.d[1], x, dim.n[1], dim.inv[1]);
+    float fz = cpr_coord_d(R.p[2], R.d[2], x, dim.n[2], dim.inv[2]);
     // "fz = 1.0 - fz" in double, then rounded to float: the float
     // subtraction rounds the same exact difference once
     if (!invertZ) fz = 1.0f - fz;
@@ -85,9 +100,11 @@ int fill_plane_params(const VolumeState &v, const mk_plane_params *p, PlaneParam
     }
     P.W = p->width;
     P.H = p->height;
+    P.fast = 1;
     for (int k = 0; k < 3; ++k) {
-        P.sp[k] = p->spacing[k];
-        P.fdim[k] = (float)v.dims[k];
+        P.ext[k] = p->spacing[k] * (float)v.dims[k];
+        P.inv_ext[k] = 1.0f / P.ext[k];
+        if (!div_by_ok(P.ext[k])) P.fast = 0;
         P.h[k] = p->dir_h[k];
         P.v[k] = p->dir_v[k];
         P.n[k] = p->dir_n[k];
@@ -242,8 +259,7 @@ extern "C" int mk_render_cpr(mk_volume vol, int width, int height, const double 
     MK_CUDA_TRY(cudaMemcpyAsync(d_rows, v.h_pinned, row_bytes, cudaMemcpyHostToDevice, s));
     short *dst = out_on_device ? out : static_cast<short *>(v.d_out);
     dim3 grid((width + 31) / 32, (height + 7) / 8);
-    const float3 fdim = make_float3((float)v.dims[0], (float)v.dims[1], (float)v.dims[2]);
-    k_cpr<<<grid, 256, 0, s>>>(width, height, fdim, invert_z ? 1 : 0, d_rows, v.tex_linear, dst);
+    k_cpr<<<grid, 256, 0, s>>>(width, height, cpr_dims(v), invert_z ? 1 : 0, d_rows, v.tex_linear, dst);
     MK_CUDA_TRY(cudaGetLastError());
     if (out_on_device) {
         // the row table in the staging buffer must outlive the kernel
@@ -323,8 +339,7 @@ extern "C" int mk_render_cpr_noalloc(mk_volume vol, int width, int height, const
     MK_CUDA_TRY(cudaMemcpyAsync(d_rows, g_noalloc_rows_host, (size_t)height * sizeof(CprRow),
                                 cudaMemcpyHostToDevice, s));
     dim3 grid((width + 31) / 32, (height + 7) / 8);
-    const float3 fdim = make_float3((float)v.dims[0], (float)v.dims[1], (float)v.dims[2]);
-    k_cpr<<<grid, 256, 0, s>>>(width, height, fdim, invert_z ? 1 : 0, d_rows, v.tex_linear, out_device);
+    k_cpr<<<grid, 256, 0, s>>>(width, height, cpr_dims(v), invert_z ? 1 : 0, d_rows, v.tex_linear, out_device);
     MK_CUDA_TRY(cudaGetLastError());
     return MK_OK;
 }
