@@ -19,9 +19,9 @@
 //    per resident slot of the device, each pulling tiles with an atomic
 //    counter until the list is exhausted (no waiting on other blocks or on
 //    the host).  A request spans steps when it has more tiles than a step
-//    takes; requests admitted meanwhile join the next step.  Steps alternate
-//    between two streams, so the next step's tiles fill the tail of the one
-//    before (a step ends with its slowest tile); up to four are in flight.
+//    takes; requests admitted meanwhile join the next step.  Steps take turns on
+//    several streams, so later steps' tiles fill the tail of the ones before
+//    (a step ends with its slowest tile).
 //    Finished images go back on a copy stream behind the steps that hold
 //    their tiles.
 #include <cuda_runtime.h>
@@ -63,12 +63,22 @@ struct SlotDesc {
     void *out;
 };
 
+// Streams that steps take in turn, and steps in flight.  A step ends with its
+// slowest tile, and the next step on its stream starts after that, so several
+// streams keep the SMs filled: a burst of 16 mixed requests takes 4.1 / 3.7 /
+// 3.6 ms (three seeds) with two streams, 4.2 / 3.2 / 3.1 with four, 3.7 / 2.9 /
+// 2.8 with six and four blocks of k_serve per SM (3.9 / 3.1 / 2.9 with three);
+// eight and twelve gain no more.
+constexpr int kStepStreams = 6;
+constexpr size_t kStepsInFlight = 6;
+constexpr int kServeBlocksPerSm = 4;
+
 struct TileItem {
     unsigned short slot, tx, ty, pad;
 };
 
 // queue layout: int count, int pad, TileItem items[count]
-__global__ void __launch_bounds__(256, 3) k_serve(const SlotDesc *__restrict__ slots, const int *__restrict__ queue,
+__global__ void __launch_bounds__(256, kServeBlocksPerSm) k_serve(const SlotDesc *__restrict__ slots, const int *__restrict__ queue,
                                                int *__restrict__ next) {
     __shared__ LabelSmem S;
     __shared__ RayParams s_rp;
@@ -188,17 +198,17 @@ struct mk_server_s {
     mk_server_config cfg;
     int blocks = 0;
     cudaStream_t stream = nullptr;                 // admissions: tables, descriptors, brick visibility
-    cudaStream_t step_stream[2] = {};              // steps alternate, so one fills the other's tail
+    cudaStream_t step_stream[kStepStreams] = {};   // steps take turns, so that later ones fill a tail
     cudaStream_t copy_stream = nullptr;            // finished images to the host
     cudaEvent_t uploaded = nullptr;                // after the latest admissions
     bool uploads_pending = false;
-    cudaEvent_t last_kernel[2] = {};               // latest step kernel on each step stream
+    cudaEvent_t last_kernel[kStepStreams] = {};               // latest step kernel on each step stream
     std::vector<Slot> slots;
     SlotDesc *d_slots = nullptr, *h_slots = nullptr;
-    int *d_queue[2] = {}, *h_queue[2] = {}, *d_next[2] = {};
-    cudaGraph_t graph[2] = {};
-    cudaGraphExec_t graph_exec[2] = {};
-    cudaEvent_t queue_free[2] = {};
+    int *d_queue[kStepStreams] = {}, *h_queue[kStepStreams] = {}, *d_next[kStepStreams] = {};
+    cudaGraph_t graph[kStepStreams] = {};
+    cudaGraphExec_t graph_exec[kStepStreams] = {};
+    cudaEvent_t queue_free[kStepStreams] = {};
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> event_pool;
     int max_items = 0;
     size_t slot_bytes = 0, resident = 0, budget = 0;
@@ -234,7 +244,7 @@ struct mk_server_s {
 namespace {
 
 void release(mk_server_s *s) {
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kStepStreams; ++b) {
         if (s->graph_exec[b]) cudaGraphExecDestroy(s->graph_exec[b]);
         if (s->graph[b]) cudaGraphDestroy(s->graph[b]);
         if (s->d_queue[b]) cudaFree(s->d_queue[b]);
@@ -265,7 +275,7 @@ void release(mk_server_s *s) {
     for (auto &kv : s->volumes) mk_volume_destroy(kv.second.vol);
     if (s->uploaded) cudaEventDestroy(s->uploaded);
     if (s->stream) cudaStreamDestroy(s->stream);
-    for (int b = 0; b < 2; ++b)
+    for (int b = 0; b < kStepStreams; ++b)
         if (s->step_stream[b]) cudaStreamDestroy(s->step_stream[b]);
     if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
 }
@@ -382,8 +392,8 @@ int admit(mk_server_s *s, uint64_t ticket, int slot_index) {
 // List the next tiles, launch the step graph and queue the copies of the
 // images it finishes (lock held).
 int issue_step(mk_server_s *s) {
-    const int b = (int)(s->step_count & 1);
-    MK_CUDA_TRY(cudaEventSynchronize(s->queue_free[b]));   // the copy of this list two steps ago is done
+    const int b = (int)(s->step_count % kStepStreams);
+    MK_CUDA_TRY(cudaEventSynchronize(s->queue_free[b]));   // this list's last copy is done
     TileItem *items = reinterpret_cast<TileItem *>(s->h_queue[b] + 2);
     int n = 0;
     Step st;
@@ -422,9 +432,10 @@ int issue_step(mk_server_s *s) {
     st.copies_done = ev.second;
     MK_CUDA_TRY(cudaEventRecord(st.kernel_done, ss));
     // A finishing request's earlier tiles are in earlier steps: those on this
-    // stream are ordered before this one, the other stream's latest may still run.
+    // stream are ordered before this one, the other streams' latest may still run.
     MK_CUDA_TRY(cudaStreamWaitEvent(s->copy_stream, st.kernel_done, 0));
-    MK_CUDA_TRY(cudaStreamWaitEvent(s->copy_stream, s->last_kernel[b ^ 1], 0));
+    for (int o = 0; o < kStepStreams; ++o)
+        if (o != b) MK_CUDA_TRY(cudaStreamWaitEvent(s->copy_stream, s->last_kernel[o], 0));
     MK_CUDA_TRY(cudaEventRecord(s->last_kernel[b], ss));
     for (uint64_t t : st.finishing) {
         Req &q = s->reqs[t];
@@ -523,8 +534,8 @@ void worker_loop(mk_server_s *s) {
             s->active.push_back(t);
             progressed = true;
         }
-        // 3. keep up to four steps in flight
-        if (rc == MK_OK && s->inflight.size() < 4) {
+        // 3. keep steps in flight
+        if (rc == MK_OK && s->inflight.size() < kStepsInFlight) {
             bool work = false;
             for (uint64_t t : s->active) {
                 const Req &q = s->reqs[t];
@@ -770,7 +781,7 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
     s->max_items = c.tiles_per_step;
     const size_t L = (size_t)c.lut_len;
     s->slot_bytes = (size_t)c.max_slots * ((size_t)c.max_labels * L * 20 + (size_t)c.max_bricks * 4 + (size_t)c.max_pixels * 4 + sizeof(SlotDesc)) +
-                    2 * (8 + (size_t)s->max_items * sizeof(TileItem));
+                    kStepStreams * (8 + (size_t)s->max_items * sizeof(TileItem));
     if (s->slot_bytes > s->budget) {
         set_last_error("mk_server_create: the slot buffers alone exceed the HBM budget");
         delete s;
@@ -783,8 +794,9 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
     AllocInjector dev_alloc;
     do {
         if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess) break;
-        if ((e = cudaStreamCreateWithFlags(&s->step_stream[0], cudaStreamNonBlocking)) != cudaSuccess) break;
-        if ((e = cudaStreamCreateWithFlags(&s->step_stream[1], cudaStreamNonBlocking)) != cudaSuccess) break;
+        for (int b = 0; b < kStepStreams && e == cudaSuccess; ++b)
+            e = cudaStreamCreateWithFlags(&s->step_stream[b], cudaStreamNonBlocking);
+        if (e != cudaSuccess) break;
         if ((e = cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) break;
         if ((e = cudaEventCreateWithFlags(&s->uploaded, cudaEventDisableTiming)) != cudaSuccess) break;
         if ((e = cudaEventRecord(s->uploaded, s->stream)) != cudaSuccess) break;
@@ -817,7 +829,7 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
         if ((e = dev_alloc((void **)&s->d_slots, c.max_slots * sizeof(SlotDesc))) != cudaSuccess) break;
         if ((e = cudaMallocHost(&s->h_slots, c.max_slots * sizeof(SlotDesc))) != cudaSuccess) break;
         const size_t qbytes = 8 + (size_t)s->max_items * sizeof(TileItem);
-        for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
+        for (int b = 0; b < kStepStreams && e == cudaSuccess; ++b) {
             if ((e = dev_alloc((void **)&s->d_queue[b], qbytes)) != cudaSuccess) break;
             if ((e = cudaMallocHost(&s->h_queue[b], qbytes)) != cudaSuccess) break;
             if ((e = dev_alloc((void **)&s->d_next[b], sizeof(int))) != cudaSuccess) break;
@@ -827,7 +839,7 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
             e = cudaEventRecord(s->last_kernel[b], s->step_stream[b]);
         }
         if (e != cudaSuccess) break;
-        for (int i = 0; i < 8 && e == cudaSuccess; ++i) {
+        for (size_t i = 0; i < 2 * kStepsInFlight && e == cudaSuccess; ++i) {
             cudaEvent_t a = nullptr, b2 = nullptr;
             if ((e = cudaEventCreateWithFlags(&a, cudaEventDisableTiming)) != cudaSuccess) break;
             if ((e = cudaEventCreateWithFlags(&b2, cudaEventDisableTiming)) != cudaSuccess) {
@@ -842,7 +854,7 @@ extern "C" int mk_server_create(const mk_server_config *config, mk_server *out) 
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device)) != cudaSuccess) break;
         s->blocks = std::max(1, per_sm) * sms;
         // one graph per queue buffer: reset the tile counter, run the persistent kernel
-        for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
+        for (int b = 0; b < kStepStreams && e == cudaSuccess; ++b) {
             cudaStream_t cap = nullptr;
             if ((e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)) != cudaSuccess) break;
             e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -888,8 +900,7 @@ extern "C" int mk_server_destroy(mk_server s) {
     if (s->encoder.joinable()) s->encoder.join();
     cudaSetDevice(s->cfg.device);
     cudaStreamSynchronize(s->stream);
-    cudaStreamSynchronize(s->step_stream[0]);
-    cudaStreamSynchronize(s->step_stream[1]);
+    for (int b = 0; b < kStepStreams; ++b) cudaStreamSynchronize(s->step_stream[b]);
     cudaStreamSynchronize(s->copy_stream);
     release(s);
     delete s;
