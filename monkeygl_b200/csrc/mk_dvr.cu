@@ -1176,40 +1176,54 @@ static BrickLayout brick_layout(const int dims[3], bool gradients) {
     return l;
 }
 
-// Whether these views gain from bricks, and may use them.  A view has about
-// W * H * 0.5 / step samples.  Measured at a quarter of a sample per voxel (one
-// view of 128^2, 256^3, plain / bricks): forward 426 / 122 us where most is
-// transparent, 426 / 377 us where all is visible; backward 1256 / 734 and 1369
-// / 1312 us.  At a sixteenth the visible case turns (backward 1245 / 1401 us).
-// Below about five million samples the rays must also be long (150 steps of
-// the ray parameter) for the shorter chain of a ray to outweigh three to six
-// more launches: a training step of 40^3 (depth 57) 236 / 296 us, of 90^3
-// (depth 129) 455 / 451 us, of 128^3 (depth 183) 586 / 450 us; eight 128^2
-// views of 64^3 (six million samples) 644 / 473 us.  The exit model of a ray (linear in the sample number) holds to a few hundredths of a
-// cell while a unit of the ray parameter is at most 3e4 cells along an axis;
-// quads are addressed with 32 bits.
+// Whether these views gain from bricks, and may use them.  Measured at a
+// quarter of a sample per voxel (one view of 128^2, 256^3, plain / bricks):
+// forward 426 / 122 us where most is transparent, 426 / 377 us where all is
+// visible; backward 1256 / 734 and 1369 / 1312 us.  At a sixteenth the visible
+// case turns (backward 1245 / 1401 us).  Below about five million samples the
+// rays must also be long for the shorter chain of a ray to outweigh three to
+// six more launches (240 samples; a forward alone of 183x96x116 with rays of
+// 220: 93 / 102 us, a training step of 40^3, 57: 236 / 296 us, of 128^3, 260:
+// 640 / 460 us; eight 128^2 views of 64^3, six million samples: 644 / 473 us),
+// and for the backward the LUT must have 64 entries: with a few, long runs in
+// one LUT cell make the plain one cheap (16 entries, 249x73x51, rays of 250:
+// 215 / 316 us a step).  The exit model
+// of a ray (linear in the sample number) holds to a few hundredths of a cell
+// while a unit of the ray parameter is at most 3e4 cells along an axis; quads
+// are addressed with 32 bits.
 constexpr double kDvrSamplesPerVoxel = 0.25;
 constexpr double kDvrManySamples = 5.0e6;
-constexpr double kDvrLongRay = 150.0;
+constexpr double kDvrLongRay = 240.0;
+constexpr int kDvrLongLut = 64;
 constexpr double kDvrMaxCellsPerUnit = 3.0e4;
 
-static bool use_bricks(const mk_dvr_params *views, int nviews) {
+static bool use_bricks(const mk_dvr_params *views, int nviews, bool backward) {
     const mk_dvr_params &a = views[0];
     double samples = 0.0, depth = 0.0;
     for (int i = 0; i < nviews; ++i) {
         const mk_dvr_params &p = views[i];
-        samples += (double)p.width * p.height * 0.5 / p.step;
-        depth = fmax(depth, 1.0 / p.step);
+        double across = 1.732;           // the longest way through the volume, in the ray parameter
         for (int k = 0; k < 3; ++k) {
-            const double unit = fabs((double)p.transform[3 * k + 1] * p.scale * p.max_len_spacing[k]) * a.dims[k];
-            if (!(unit <= kDvrMaxCellsPerUnit)) return false;
+            const double unit = fabs((double)p.transform[3 * k + 1] * p.scale * p.max_len_spacing[k]);
+            if (!(unit * a.dims[k] <= kDvrMaxCellsPerUnit)) return false;
+            if (unit > 0.0) across = fmin(across, 1.0 / unit);
         }
+        // half of that for every pixel, and at most the box's volume in (u, v,
+        // ray parameter) over that of a sample
+        const float *m = p.transform;
+        const double det = fabs((double)m[0] * ((double)m[4] * m[8] - (double)m[5] * m[7]) -
+                                (double)m[1] * ((double)m[3] * m[8] - (double)m[5] * m[6]) +
+                                (double)m[2] * ((double)m[3] * m[7] - (double)m[4] * m[6]));
+        const double mls = fabs((double)p.max_len_spacing[0] * p.max_len_spacing[1] * p.max_len_spacing[2]);
+        const double box = (double)p.height * p.height / (p.scale * det * mls);
+        samples += fmin((double)p.width * p.height * 0.5 * across, box) / p.step;
+        depth = fmax(depth, across / p.step);
     }
     for (int k = 0; k < 3; ++k)
         if (a.dims[k] > 4096) return false;
     const BrickLayout l = brick_layout(a.dims, false);
     if (l.nb[1] > 65535 || l.nb[2] > 65535 || l.n * kDvrBrickQuads >= 0xffffffffull) return false;
-    if (samples < kDvrManySamples && depth < kDvrLongRay) return false;
+    if (samples < kDvrManySamples && (depth < kDvrLongRay || (backward && a.lut_len < kDvrLongLut))) return false;
     return samples >= kDvrSamplesPerVoxel * a.dims[0] * a.dims[1] * (double)a.dims[2];
 }
 
@@ -1259,8 +1273,9 @@ static void launch_forward_bricks(const DvrBatch &B, const DvrBricks &K, int vie
 }
 
 // Scratch the caller gave, if it is enough and aligned for these views.
-static bool bricks_fit(const mk_dvr_params *views, int nviews, bool gradients, const void *scratch, size_t bytes) {
-    return scratch && (reinterpret_cast<uintptr_t>(scratch) & 255) == 0 && use_bricks(views, nviews) &&
+static bool bricks_fit(const mk_dvr_params *views, int nviews, bool backward, bool gradients, const void *scratch,
+                       size_t bytes) {
+    return scratch && (reinterpret_cast<uintptr_t>(scratch) & 255) == 0 && use_bricks(views, nviews, backward) &&
            bytes >= brick_layout(views[0].dims, gradients).bytes;
 }
 
@@ -1288,7 +1303,7 @@ extern "C" int mk_dvr_scratch_bytes(const mk_dvr_params *views, int nviews, int 
     }
     int rc = check_views(views, nviews);
     if (rc != MK_OK) return rc;
-    *bytes = use_bricks(views, nviews) ? brick_layout(views[0].dims, gradients != 0).bytes : 0;
+    *bytes = use_bricks(views, nviews, gradients != 0) ? brick_layout(views[0].dims, gradients != 0).bytes : 0;
     return MK_OK;
 }
 
@@ -1304,7 +1319,7 @@ extern "C" int mk_dvr_forward_scratch(const mk_dvr_params *views, int nviews, co
     cudaStream_t s = (cudaStream_t)stream;
     const size_t npix = (size_t)views[0].width * views[0].height;
     const size_t smem = 2 * (size_t)views[0].lut_len * sizeof(float4);
-    const bool bricks = bricks_fit(views, nviews, false, scratch, scratch_bytes);
+    const bool bricks = bricks_fit(views, nviews, false, false, scratch, scratch_bytes);
     DvrBricks K = {};
     if (bricks) {
         rc = build_bricks<false>(views[0], volume, lut, scratch, false, K, s);
@@ -1344,7 +1359,7 @@ extern "C" int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, c
     if (rc != MK_OK) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t npix = (size_t)views[0].width * views[0].height;
-    const bool bricks = bricks_fit(views, nviews, grad_volume != nullptr, scratch, scratch_bytes);
+    const bool bricks = bricks_fit(views, nviews, true, grad_volume != nullptr, scratch, scratch_bytes);
     const size_t smem = 3 * (size_t)views[0].lut_len * sizeof(float4), smem_b = smem + kWin * kBackThreads * sizeof(float4);
     DvrBricks K = {};
     double *lut_sums = nullptr;

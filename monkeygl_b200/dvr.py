@@ -59,12 +59,13 @@ def _check(rc, where):
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def view_array(views):
     """The views as a C array of DVRParams (ctypes)."""
-    views = list(views)
+    if not isinstance(views, list):
+        views = list(views)
     return (DVRParams * len(views))(*views), len(views)
 
 
@@ -100,12 +101,17 @@ def _torch_function():
             L = _lib()
             arr, nv = view_array(views)
             p0 = arr[0]
-            for p in arr:
-                if p.lut_len != lut.shape[0] or tuple(p.dims) != tuple(volume.shape[::-1]):
+            if p0.lut_len != lut.shape[0] or tuple(p0.dims) != tuple(volume.shape[::-1]):
+                raise ValueError("view parameters do not match the volume or LUT")
+            # the other views share the first one's size, dims and LUT length
+            # (compared as bytes: a ctypes field costs more than a small launch)
+            raw, n = memoryview(arr).cast("B"), C.sizeof(DVRParams)
+            for o in range(n, len(raw), n):
+                if raw[o + 8:o + 20] != raw[8:20] or raw[o + n - 4:o + n] != raw[n - 4:n]:
                     raise ValueError("view parameters do not match the volume or LUT")
-                if (p.width, p.height) != (p0.width, p0.height):
+                if raw[o:o + 8] != raw[:8]:
                     raise ValueError("the views of one render must share width and height")
-            stream = C.c_void_p(torch.cuda.current_stream(volume.device).cuda_stream)
+            stream = torch.cuda.current_stream(volume.device).cuda_stream
             images = torch.empty((nv, p0.height, p0.width, 3), dtype=torch.float32, device=volume.device)
             trans = torch.empty((nv, p0.height, p0.width), dtype=torch.float32, device=volume.device)
             work = None
@@ -123,7 +129,7 @@ def _torch_function():
         def backward(ctx, grad_images):
             volume, lut = ctx.saved_tensors
             L = _lib()
-            stream = C.c_void_p(torch.cuda.current_stream(volume.device).cuda_stream)
+            stream = torch.cuda.current_stream(volume.device).cuda_stream
             grad_lut = torch.zeros_like(lut)
             grad_vol = torch.zeros_like(volume) if ctx.needs_input_grad[0] else None
             g = grad_images.contiguous().float()

@@ -83,15 +83,15 @@ def _close(a, b):
 
 
 @pytest.mark.parametrize("dims,size,views,lut,kind,step,t_min", [
-    ((9, 8, 17), (20, 12), 1, 16, "cut", 0.1, 1e-4),
-    ((7, 7, 7), (9, 7), 2, 2, "seen", 0.04, 0.0),
-    ((1, 24, 33), (31, 17), 3, 64, "seen", 0.2, 0.0),
-    ((40, 31, 50), (65, 47), 4, 256, "cut", 0.3, 1e-4),
-    ((40, 31, 50), (65, 47), 2, 256, "opaque", 0.33, 0.0),
-    ((64, 64, 64), (78, 75), 33, 1000, "cut", 1.0, 0.05),
-    ((48, 56, 64), (400, 380), 2, 128, "seen", 0.5, 1e-3),
-    ((32, 32, 32), (24, 24), 1, 32, "cut", 0.2, 2.0),
-    ((170, 165, 168), (160, 150), 1, 64, "cut", 0.7, 1e-3),
+    ((9, 8, 17), (20, 12), 1, 64, "cut", 0.02, 1e-4),
+    ((7, 7, 7), (9, 7), 2, 64, "seen", 0.02, 0.0),
+    ((1, 24, 33), (31, 17), 3, 64, "seen", 0.004, 0.0),
+    ((40, 31, 50), (65, 47), 4, 256, "cut", 0.12, 1e-4),
+    ((40, 31, 50), (65, 47), 2, 256, "opaque", 0.13, 0.0),
+    ((64, 64, 64), (110, 105), 33, 1000, "cut", 1.0, 0.05),
+    ((48, 56, 64), (400, 380), 2, 2, "seen", 0.3, 1e-3),
+    ((32, 32, 32), (24, 24), 1, 100, "cut", 0.1, 2.0),
+    ((170, 165, 168), (160, 150), 1, 64, "cut", 0.5, 1e-3),
 ])
 def test_bricks_match_plain(dims, size, views, lut, kind, step, t_min):
     vol, table = _volume(dims, 3), _lut(lut, kind, 4)
@@ -110,7 +110,7 @@ def test_bricks_match_plain(dims, size, views, lut, kind, step, t_min):
 def test_gradients_that_are_not_finite_spread_as_before():
     dims, n = (40, 31, 50), 64
     vol, table = _volume(dims, 6), _lut(n, "cut", 7)
-    vs = _views(2, 33, 29, dims, n, 0.3, 1e-4)
+    vs = _views(2, 33, 29, dims, n, 0.12, 1e-4)
     g = torch.randn((2, 29, 33, 3), generator=torch.Generator("cuda").manual_seed(8), device="cuda")
     g[0, 14, 16, 1] = float("inf")
     g[1, 10, 12, 0] = float("nan")
@@ -124,10 +124,10 @@ def test_gradients_that_are_not_finite_spread_as_before():
 def test_values_outside_the_unit_range():
     """Voxels beyond what the range test of a brick can place (and NaN) are
     rendered, not left out."""
-    dims, n = (24, 24, 24), 32
+    dims, n = (24, 24, 24), 64
     vol, table = _volume(dims, 9), _lut(n, "cut", 10)
     vol[5, 5, 5], vol[12, 12, 12], vol[18, 9, 9] = 1e30, float("nan"), -50.0
-    vs = _views(1, 40, 40, dims, n, 0.15, 0.0)
+    vs = _views(1, 40, 40, dims, n, 0.08, 0.0)
     g = torch.ones((1, 40, 40, 3), device="cuda")
     a, b = (_run(vs, vol, table, g, bricks, True) for bricks in (False, True))
     assert torch.equal(a[0], b[0]) and torch.equal(a[2], b[2])
