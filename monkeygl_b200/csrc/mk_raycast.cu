@@ -214,21 +214,27 @@ static void launch_raycast(int mode, int track, const RayParams &P, cudaTextureO
     }
 }
 
-// Tiles still unfinished when rays start to spill to the tail launch:
-// two thirds of the SM count (measured on 1024^2 body frames on 148 SMs:
-// 16, 48, 96, 148, 296 tiles gave 2699, 2907, 2989, 2761, 2445 frames/s).
+// Tiles still unfinished when rays start to spill to the tail launch: the SM
+// count for frames of ten tiles per SM and more, two thirds of it below.
+// Measured on 148 SMs with 64 / 98 / 148 / 222 tiles, microseconds a frame, sums
+// over four volumes: 1024^2 (4096 tiles) 1253 / 1227 / 1209 / 1208 (labelled
+// 512x512x1559: 198 / 191 / 177 / 177), 640^2 967 / 923 / 918 / 1036, 512^2
+// (1024 tiles) 897 / 874 / 906 / 1149, 384^2 772 / 757 / 833 / 1001.
 // MONKEYGL_B200_TAIL_TILES overrides it (0: rays never spill).
-static int tail_tiles() {
-    static const int k = [] {
+static int tail_tiles(int ntiles) {
+    static const int forced = [] {
         const char *e = getenv("MONKEYGL_B200_TAIL_TILES");
-        if (e) return std::max(0, atoi(e));
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            sms = 148;
-        return std::max(1, 2 * sms / 3);
+        return e ? std::max(0, atoi(e)) : -1;
     }();
-    return k;
+    static const int sms = [] {
+        int dev = 0, n = 148;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            n = 148;
+        return n;
+    }();
+    if (forced >= 0) return forced;
+    return std::max(1, ntiles >= 10 * sms ? sms : 2 * sms / 3);
 }
 
 // The tail buffers of stream s (created on first use, grown for larger
@@ -236,7 +242,7 @@ static int tail_tiles() {
 // their own; a fifth renders without a tail launch.
 static int tail_params(VolumeState &v, RayParams &P, cudaStream_t s) {
     const int ntiles = ((P.W + 31) / 32) * ((P.H + 7) / 8);
-    const int K = tail_tiles();
+    const int K = tail_tiles(ntiles);
     if (K == 0) return MK_OK;                      // no hand-off: P.tail stays null
     const int want = (int)std::min<long long>((long long)P.W * P.H, std::max(4LL * K * 256, 65536LL));
     int i = 0;
