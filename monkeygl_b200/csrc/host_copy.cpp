@@ -15,9 +15,9 @@
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
+#include <exception>
 #include <mutex>
 #include <new>
-#include <system_error>
 #include <thread>
 
 #include "mk_internal.h"
@@ -44,23 +44,25 @@ struct CopyPool {
     std::mutex mu;
     std::condition_variable cv;
     uint64_t wakes = 0;                      // guarded by mu
-    // generation of the copy (high 32 bits) and its next piece; a piece is
-    // taken by advancing it under the same generation
+    // generation of the copy (high 32 bits) and its pieces not yet taken: a
+    // piece is taken by counting one down under the same generation.  Between
+    // copies none are left, so a helper that is late for one copy cannot take
+    // a piece of the next, whose size it would otherwise see too early.
     std::atomic<uint64_t> ticket{0};
     std::atomic<uint32_t> done{0};
-    char *dst = nullptr;
+    char *dst = nullptr;                     // written only while no piece is left
     const char *src = nullptr;
     size_t bytes = 0;
-    std::atomic<uint32_t> pieces{0};
 
     bool take(uint32_t gen) {
         uint64_t t = ticket.load(std::memory_order_acquire);
         for (;;) {
-            if ((uint32_t)(t >> 32) != gen || (uint32_t)t >= pieces.load(std::memory_order_relaxed)) return false;
-            if (ticket.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel, std::memory_order_acquire)) break;
+            if ((uint32_t)(t >> 32) != gen || (uint32_t)t == 0) return false;
+            if (ticket.compare_exchange_weak(t, t - 1, std::memory_order_acq_rel, std::memory_order_acquire)) break;
         }
         // the piece is this thread's, and the copy cannot end without it
-        const size_t off = (size_t)(uint32_t)t * kPiece;
+        const uint32_t n = (uint32_t)((bytes + kPiece - 1) / kPiece);
+        const size_t off = (size_t)(n - (uint32_t)t) * kPiece;
         memcpy(dst + off, src + off, std::min(kPiece, bytes - off));
         done.fetch_add(1, std::memory_order_release);
         return true;
@@ -68,7 +70,6 @@ struct CopyPool {
 
     void helper() {
         uint64_t seen = 0;
-        uint32_t gen = 0;
         for (;;) {
             {
                 std::unique_lock<std::mutex> lk(mu);
@@ -77,10 +78,9 @@ struct CopyPool {
             }
             const auto until = std::chrono::steady_clock::now() + kSpin;
             for (int i = 0;; ++i) {
-                const uint32_t g = (uint32_t)(ticket.load(std::memory_order_acquire) >> 32);
-                if (g != gen) {
-                    gen = g;
-                    while (take(g)) {
+                const uint64_t t = ticket.load(std::memory_order_acquire);
+                if ((uint32_t)t != 0) {
+                    while (take((uint32_t)(t >> 32))) {
                     }
                     break;
                 }
@@ -94,7 +94,7 @@ struct CopyPool {
         if (std::thread::hardware_concurrency() < 2 * (kHelpers + 1)) return;
         try {
             for (int i = 0; i < kHelpers; ++i) std::thread([this] { helper(); }).detach();
-        } catch (const std::system_error &) {    // fewer helpers, or none
+        } catch (const std::exception &) {       // fewer helpers, or none
         }
     }
 };
@@ -129,8 +129,7 @@ void copy_out(void *dst, const void *src, size_t bytes) {
     p->src = static_cast<const char *>(src);
     p->bytes = bytes;
     p->done.store(0, std::memory_order_relaxed);
-    p->pieces.store(n, std::memory_order_relaxed);
-    p->ticket.store((uint64_t)gen << 32, std::memory_order_release);
+    p->ticket.store((uint64_t)gen << 32 | n, std::memory_order_release);
     while (p->take(gen)) {
     }
     while (p->done.load(std::memory_order_acquire) != n) pause_cpu();

@@ -27,7 +27,24 @@ static bool many(unsigned seed) {
     return ok;
 }
 
+// Copies close together, each larger than the one before: helpers are late for
+// one and meet the next.
+static bool close_together() {
+    std::vector<unsigned char> src(786432), dst(786432);
+    for (size_t i = 0; i < src.size(); ++i) src[i] = (unsigned char)((i * 2654435761u) >> 13);
+    for (int r = 0; r < 20000; ++r) {
+        const size_t n = 262144 + (size_t)(r % 9) * 65536;
+        dst[n - 1] = (unsigned char)~src[n - 1];
+        mk::copy_out_soon(n);
+        mk::copy_out(dst.data(), src.data(), n);
+        if (dst[n - 1] != src[n - 1] || dst[0] != src[0]) return false;
+        dst[0] = (unsigned char)~src[0];
+    }
+    return memcmp(dst.data() + 1, src.data() + 1, dst.size() - 1) == 0;
+}
+
 int main() {
+    if (!close_together()) return printf("close together\n"), 1;
     if (!many(1)) return printf("one thread\n"), 1;
     bool ok[6];
     std::vector<std::thread> ts;
