@@ -187,23 +187,29 @@ __device__ __forceinline__ bool outside_voi(const RayParams &P, const float3 &x)
            x.z >= P.voi_hi[2];
 }
 
-// The brick of a sample, clamped to the volume, and its position in bricks
+// The brick of a sample, clamped to the volume, and its position in voxels
 // with the brick's corner (unclamped: the neighbour of an edge brick where a
 // position lies outside the volume, which is as empty as the edge brick).
+// Floats about kBrickMagic are a brick's edge apart, so a sum with it rounded
+// down gives the corner, and its low bits the brick's index.
 constexpr float kFloorMagic = 12582912.0f;      // 0x4b400000
+constexpr float kBrickMagic = kBrick * kFloorMagic;
+constexpr uint32_t kBrickMagicBits = 0x4b400000u + (kBrickShift << 23);
 struct BrickPos {
-    float3 q, lo;
+    float3 x, lo;
     int b;
 };
 
+__device__ __forceinline__ int brick_bits(float t) { return (int)(__float_as_uint(t) - kBrickMagicBits); }
+
 __device__ __forceinline__ BrickPos brick_pos(const RayParams &P, const BrickView &BV, const float3 &x) {
     BrickPos r;
-    r.q = make_float3(x.x * 0.125f, x.y * 0.125f, x.z * 0.125f);
-    const float tx = __fadd_rd(r.q.x, kFloorMagic), ty = __fadd_rd(r.q.y, kFloorMagic), tz = __fadd_rd(r.q.z, kFloorMagic);
-    r.lo = make_float3(tx - kFloorMagic, ty - kFloorMagic, tz - kFloorMagic);
-    const int ix = min(max(__float_as_int(tx) - 0x4b400000, 0), BV.nbx - 1);
-    const int iy = min(max(__float_as_int(ty) - 0x4b400000, 0), BV.nby - 1);
-    const int iz = min(max(__float_as_int(tz) - 0x4b400000, 0), BV.nbz - 1);
+    r.x = x;
+    const float tx = __fadd_rd(x.x, kBrickMagic), ty = __fadd_rd(x.y, kBrickMagic), tz = __fadd_rd(x.z, kBrickMagic);
+    r.lo = make_float3(tx - kBrickMagic, ty - kBrickMagic, tz - kBrickMagic);
+    const int ix = min(max(brick_bits(tx), 0), BV.nbx - 1);
+    const int iy = min(max(brick_bits(ty), 0), BV.nby - 1);
+    const int iz = min(max(brick_bits(tz), 0), BV.nbz - 1);
     r.b = (iz * BV.nby + iy) * BV.nbx + ix;
     return r;
 }
@@ -217,24 +223,24 @@ __device__ __forceinline__ int label_at(cudaTextureObject_t mask, const float3 &
     return min((int)tex3D<unsigned char>(mask, fx, fy, fz), MK_MAX_LABELS - 1);
 }
 
-// A ray's way through bricks: coarse steps per brick along each axis, and the
-// position in a brick (of edge 1, 0.05 voxels of margin) at which it leaves;
-// an axis it does not move along never ends a run.
+// A ray's way through bricks: coarse steps per voxel along each axis, and the
+// position in a brick (with 0.05 voxels of margin) at which it leaves; an axis
+// it does not move along never ends a run.
 struct StepVec {
     float3 rd, off;
 };
 
 __device__ __forceinline__ StepVec step_vec(const RayParams &P) {
     StepVec S;
-    const float ds = P.step1 * P.scale, e = 0.05f / kBrick;
+    const float ds = P.step1 * P.scale, e = 0.05f;
     const float d[3] = {P.M[1] * P.mls[0] * ds * P.fdim[0], P.M[4] * P.mls[1] * ds * P.fdim[1],
                         (P.invertZ ? -P.M[7] : P.M[7]) * P.mls[2] * ds * P.fdim[2]};
     float rd[3], off[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const bool moves = fabsf(d[k]) > 1e-6f;
-        rd[k] = moves ? (float)kBrick / d[k] : 1.0f;
-        off[k] = !moves ? 1e9f : d[k] > 0.0f ? 1.0f - e : e;
+        rd[k] = moves ? 1.0f / d[k] : 1.0f;
+        off[k] = !moves ? 1e9f : d[k] > 0.0f ? kBrick - e : e;
     }
     S.rd = make_float3(rd[0], rd[1], rd[2]);
     S.off = make_float3(off[0], off[1], off[2]);
@@ -247,9 +253,10 @@ __device__ __forceinline__ StepVec step_vec(const RayParams &P) {
 // the rounding of the linear model.
 constexpr int kMaxRun = 240;
 __device__ __forceinline__ float time_in_brick(const BrickPos &p, const StepVec &sv, float reach) {
-    const float tx = __fmaf_rn(reach, fabsf(sv.rd.x), (p.lo.x - p.q.x + sv.off.x) * sv.rd.x);
-    const float ty = __fmaf_rn(reach, fabsf(sv.rd.y), (p.lo.y - p.q.y + sv.off.y) * sv.rd.y);
-    const float tz = __fmaf_rn(reach, fabsf(sv.rd.z), (p.lo.z - p.q.z + sv.off.z) * sv.rd.z);
+    const float r = kBrick * reach;
+    const float tx = __fmaf_rn(r, fabsf(sv.rd.x), (p.lo.x - p.x.x + sv.off.x) * sv.rd.x);
+    const float ty = __fmaf_rn(r, fabsf(sv.rd.y), (p.lo.y - p.x.y + sv.off.y) * sv.rd.y);
+    const float tz = __fmaf_rn(r, fabsf(sv.rd.z), (p.lo.z - p.x.z + sv.off.z) * sv.rd.z);
     return fmaxf(fminf(fminf(tx, ty), fminf(tz, (float)kMaxRun)), 0.0f);
 }
 
@@ -1072,12 +1079,14 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
 // windowed value.  CHECK: samples may lie outside the VOI.  Without it the loop
 // holds what a sample cannot do without: the position, the brick (without
 // clamping), the bound and the fetch.  Issue-bound (79% of the issue slots): 512x512x361 at
-// 1024^2 388 -> 316 us.
+// 1024^2 388 -> 316 us, and 322 -> 314 us a call with a brick's index and corner
+// from one rounded sum per axis and the test of P.skip out of the loop.
 template <bool CHECK>
 __device__ __forceinline__ int mip_entries(const RayParams &P, cudaTextureObject_t vol, const BrickView &BV,
                                            const StepVec &dv, float u, float v, int k, int end, float &vmax, float &A) {
-    const uint32_t nbx = BV.nbx, nby = BV.nby, zero = ((0x4b400000u * nby) + 0x4b400000u) * nbx + 0x4b400000u;
+    const uint32_t nbx = BV.nbx, nby = BV.nby, zero = (kBrickMagicBits * nby + kBrickMagicBits) * nbx + kBrickMagicBits;
     const uint32_t last = nbx * nby * (uint32_t)BV.nbz - 1u;   // (no index can leave the map)
+    float known = P.skip ? A : NAN;         // bricks up to it are skipped (none up to NaN)
     while (k < end) {
         const float3 pos = ray_pos_fy(P, u, v, P.fy_tab[k]);
         const float3 x = voxel_pos(P, pos);
@@ -1085,20 +1094,18 @@ __device__ __forceinline__ int mip_entries(const RayParams &P, cudaTextureObject
             ++k;
             continue;
         }
-        if (P.skip) {
-            BrickPos bp;
-            if (CHECK) {
-                bp = brick_pos(P, BV, x);
-            } else {
-                bp.q = make_float3(x.x * 0.125f, x.y * 0.125f, x.z * 0.125f);
-                const float tx = __fadd_rd(bp.q.x, kFloorMagic), ty = __fadd_rd(bp.q.y, kFloorMagic), tz = __fadd_rd(bp.q.z, kFloorMagic);
-                bp.lo = make_float3(tx - kFloorMagic, ty - kFloorMagic, tz - kFloorMagic);
-                bp.b = (int)min((__float_as_uint(tz) * nby + __float_as_uint(ty)) * nbx + __float_as_uint(tx) - zero, last);
-            }
-            if (BV.mip_tmax[bp.b] <= A) {
-                k += 1 + steps_in_brick(bp, dv);
-                continue;
-            }
+        BrickPos bp;
+        if (CHECK) {
+            bp = brick_pos(P, BV, x);
+        } else {
+            bp.x = x;
+            const float tx = __fadd_rd(x.x, kBrickMagic), ty = __fadd_rd(x.y, kBrickMagic), tz = __fadd_rd(x.z, kBrickMagic);
+            bp.lo = make_float3(tx - kBrickMagic, ty - kBrickMagic, tz - kBrickMagic);
+            bp.b = (int)min((__float_as_uint(tz) * nby + __float_as_uint(ty)) * nbx + __float_as_uint(tx) - zero, last);
+        }
+        if (BV.mip_tmax[bp.b] <= known) {
+            k += 1 + steps_in_brick(bp, dv);
+            continue;
         }
         const float raw = tex3D<float>(vol, pos.x, pos.y, pos.z);
         ++k;
@@ -1107,8 +1114,11 @@ __device__ __forceinline__ int mip_entries(const RayParams &P, cudaTextureObject
             float temp = 32768 * raw;
             temp = (temp - P.mip_wl) / P.mip_ww + 0.5f;
             if (A < temp) A = temp;
-            // the output saturates at 1.0 (core/kernel.cu:351-358)
-            if (P.skip && A >= 1.0f) break;
+            if (P.skip) {
+                known = A;
+                // the output saturates at 1.0 (core/kernel.cu:351-358)
+                if (A >= 1.0f) break;
+            }
         }
     }
     return k;
