@@ -9,7 +9,7 @@
 // nearest filtering at integer coordinates; each label's RGBA LUT is a 1D
 // float4 array read with linear filtering.  On top of that this file keeps,
 // per 8^3 brick, the voxel min/max over the brick's trilinear footprint and
-// the set of labels it owns, and rebuilds a visibility bitmap whenever a
+// the set of labels it owns, and rebuilds the VR maps and MIP bounds whenever a
 // transfer function or window changes.
 #include <cuda_runtime.h>
 #include <math.h>
