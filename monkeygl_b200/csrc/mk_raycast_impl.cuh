@@ -448,7 +448,13 @@ constexpr int kCoopEnd = 1;        // past the end of the ray (a >= limit or a >
 constexpr int kCoopOutside = 2;    // outside the VOI: no fetch
 constexpr int kCoopEmpty = 4;      // in a brick that no transfer function can show (step L1)
 constexpr int kCoopFetched = 8;    // label, value and LUT fetched
-constexpr int kCoopRaysDefault = 16;
+// Below eight lanes a ray a round costs more than the rays' own lanes would
+// take: with at most 16 / 8 / 4 / 2 rays, calls of 512^2 on 128x128x96 take 222 /
+// 218 / 217 / 216 us, 1024^2 on 512x512x361 260 / 253 / 250 / 253, labelled
+// 512x512x1559 199 / 192 / 187 / 185, its dense transfer function 1752 / 1710 /
+// 1714 / 1719, a burst of 16 served requests 3317 / 3183 / 3141 / 3119.  (Each
+// scaled by its ratio to the next; inputs differ from run to run.)
+constexpr int kCoopRaysDefault = 4;
 
 struct VrRay {
     float u, v, a, a_stop, step, aPre, A;
