@@ -510,6 +510,7 @@ __global__ void __launch_bounds__(128) k_dvr_backward(const __grid_constant__ Dv
 
 constexpr int kDvrBrickQuads = 576;      // 8 x 8 x 9
 constexpr float kDvrExitMargin = 0.05f;  // cells; covers the rounding of the linear exit model
+constexpr float kDvrSlow = 1e-4f;        // cells a sample (samples_inside)
 
 struct DvrBricks {
     int nb[3];
@@ -695,27 +696,42 @@ __device__ __forceinline__ uint32_t brick_of(const DvrBatch &B, const DvrBricks 
     return ((uint32_t)(c.z >> 3) * K.nb[1] + (c.y >> 3)) * K.nb[0] + (c.x >> 3);
 }
 
-// Further samples (in the direction of `rate`, cells per sample) certain to
-// stay in the bricks within `reach` of the one that holds cell c.
-__device__ __forceinline__ int samples_inside(const BrickCell &c, const float3 &inv, int reach) {
+// Samples per cell along each axis; 0: slower than 1e-4 cells a sample, with
+// DRIFT, or not moving at all.
+template <bool DRIFT>
+__device__ __forceinline__ float3 inverse_rate(const DvrBatch &B, const Ray &r, float step) {
+    const float x = r.dx * step * B.fdim[0], y = r.dy * step * B.fdim[1], z = r.dz * step * B.fdim[2];
+    const float slow = DRIFT ? kDvrSlow : 0.0f;
+    return make_float3(fabsf(x) > slow ? 1.0f / x : 0.0f, fabsf(y) > slow ? 1.0f / y : 0.0f,
+                       fabsf(z) > slow ? 1.0f / z : 0.0f);
+}
+
+// Further samples (after sample i in cell c, or BACK, before it) certain to stay
+// in the bricks within `reach` of the one that holds c.  DRIFT: an axis is slower
+// than kDvrSlow and yet moves (a camera turned in steps leaves 1e-8 in its
+// matrix), and a ray on a brick's face crosses it by one rounding.  So the last
+// of those samples is looked at: every operation of a coordinate is rounded
+// monotonically, so the samples between lie between.
+template <bool BACK, bool DRIFT>
+__device__ __forceinline__ int samples_inside(const DvrBatch &B, const Ray &r, float step, const float3 &inv, int i,
+                                              const BrickCell &c, int reach) {
     float t = 4096.0f;
     const int b[3] = {c.x >> 3, c.y >> 3, c.z >> 3};
     const float p[3] = {c.x + c.wx, c.y + c.wy, c.z + c.wz};
-    const float iv[3] = {inv.x, inv.y, inv.z};
+    const float iv[3] = {BACK ? -inv.x : inv.x, BACK ? -inv.y : inv.y, BACK ? -inv.z : inv.z};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float lo = (float)((b[k] - reach) * 8), hi = (float)((b[k] + reach + 1) * 8);
         const float room = iv[k] > 0.0f ? hi - kDvrExitMargin - p[k] : lo + kDvrExitMargin - p[k];
         if (iv[k] != 0.0f) t = fminf(t, room * iv[k]);
     }
-    return t > 0.0f ? (int)t : 0;
-}
-
-// Samples per cell along each axis (0: the ray does not move along it).
-__device__ __forceinline__ float3 inverse_rate(const DvrBatch &B, const Ray &r, float step) {
-    const float x = r.dx * step * B.fdim[0], y = r.dy * step * B.fdim[1], z = r.dz * step * B.fdim[2];
-    return make_float3(fabsf(x) > 1e-6f ? 1.0f / x : 0.0f, fabsf(y) > 1e-6f ? 1.0f / y : 0.0f,
-                       fabsf(z) > 1e-6f ? 1.0f / z : 0.0f);
+    const int n = t > 0.0f ? (int)t : 0;
+    if (DRIFT) {
+        const int j = BACK ? max(i - n, 0) : min(i + n, r.n - 1);
+        const BrickCell e = brick_cell(B, r, step, (float)j);
+        if (abs((e.x >> 3) - b[0]) > reach || abs((e.y >> 3) - b[1]) > reach || abs((e.z >> 3) - b[2]) > reach) return 0;
+    }
+    return n;
 }
 
 __device__ __forceinline__ float quad_trilinear(const float4 &a, const float4 &b, float wx, float wy, float wz) {
@@ -754,7 +770,7 @@ __device__ __forceinline__ DvrPixel dvr_pixel(const DvrBatch &B, int views) {
 // are k_dvr_forward's, without those that change nothing.
 constexpr int kForwardThreads = 128;
 
-template <int kAhead>
+template <int kAhead, bool DRIFT>
 __global__ void __launch_bounds__(kForwardThreads) k_dvr_forward_bricks(const __grid_constant__ DvrBatch B,
                                                             const __grid_constant__ DvrBricks K, int views,
                                                             const float4 *__restrict__ lut_g,
@@ -773,7 +789,7 @@ __global__ void __launch_bounds__(kForwardThreads) k_dvr_forward_bricks(const __
     const int cmask = (1 << V.ckpt_shift) - 1;
     float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
     const Ray r = make_ray(B, V, x, y);
-    const float3 inv = inverse_rate(B, r, V.step);
+    const float3 inv = inverse_rate<DRIFT>(B, r, V.step);
     // a threshold above 1 ends every ray at its first sample
     const bool may_skip = !(T < V.t_min);
     int i = 0, look = 0;                 // look: first sample whose brick is not known
@@ -785,7 +801,7 @@ __global__ void __launch_bounds__(kForwardThreads) k_dvr_forward_bricks(const __
             BrickCell c = brick_cell(B, r, V.step, (float)i);
             const uint32_t b = brick_of(B, K, c);
             const int d = K.dist[b];
-            look = min(i + 1 + samples_inside(c, inv, max(d - 1, 0)), r.n);
+            look = min(i + 1 + samples_inside<false, DRIFT>(B, r, V.step, inv, i, c, max(d - 1, 0)), r.n);
             brick = K.quads + (size_t)b * kDvrBrickQuads;
             if (d > 0) {
                 sample = false;
@@ -894,7 +910,7 @@ __device__ __forceinline__ void flush_quads(float4 *g, uint32_t cell, const floa
 // views of 256^2; five: 1.52).  The next sample's loads are issued before a
 // sample is summed.  Tried and left: four lanes per ray (2.26 ms; forward 1.14
 // against 0.64: the brick look-ups are then made by every lane).
-template <bool VOLGRAD>
+template <bool VOLGRAD, bool DRIFT>
 __global__ void __launch_bounds__(kBackThreads, 6)
 k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant__ DvrBricks K, int views,
                       const float4 *__restrict__ lut_g, const float *__restrict__ work,
@@ -930,8 +946,7 @@ k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant_
         if ((gr == 0.0f && gg == 0.0f && gb == 0.0f) || !gradient_finite(gr, gg, gb)) ns = 0;
     }
     const Ray r = make_ray(B, V, px.x, px.y);
-    float3 inv = inverse_rate(B, r, V.step);
-    inv = make_float3(-inv.x, -inv.y, -inv.z);
+    const float3 inv = inverse_rate<DRIFT>(B, r, V.step);
     const int cmask = (1 << V.ckpt_shift) - 1;
     float U = 0.0f;                      // U . g
     int wbase = 0;                       // first LUT cell of the window
@@ -955,7 +970,7 @@ k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant_
             const uint32_t b = brick_of(B, K, c);
             const int d = K.dist[b];
             flat = d > 0;
-            look = max(i - samples_inside(c, inv, max(d - 1, 0)), 0);
+            look = max(i - samples_inside<true, DRIFT>(B, r, V.step, inv, i, c, max(d - 1, 0)), 0);
             brick = b * kDvrBrickQuads;
             wx = c.wx;
             wy = c.wy;
@@ -1263,13 +1278,26 @@ static unsigned dvr_blocks(const DvrBatch &B, int views, int threads) {
 // cost resident warps, and 686 with one).  The line: about 2000 rays per SM.
 constexpr long long kDvrManyRays = 300000;
 
-static void launch_forward_bricks(const DvrBatch &B, const DvrBricks &K, int views, const float4 *lut, float *images,
-                                  float *trans, float *work, size_t smem, cudaStream_t s) {
-    const unsigned grid = dvr_blocks(B, views, kForwardThreads);
-    if ((long long)B.W * B.H * views >= kDvrManyRays)
-        k_dvr_forward_bricks<2><<<grid, kForwardThreads, smem, s>>>(B, K, views, lut, images, trans, work);
-    else
-        k_dvr_forward_bricks<4><<<grid, kForwardThreads, smem, s>>>(B, K, views, lut, images, trans, work);
+static void launch_forward_bricks(const DvrBatch &B, const DvrBricks &K, int views, bool drift, const float4 *lut,
+                                  float *images, float *trans, float *work, size_t smem, cudaStream_t s) {
+    const bool many = (long long)B.W * B.H * views >= kDvrManyRays;
+    auto kern = many ? (drift ? k_dvr_forward_bricks<2, true> : k_dvr_forward_bricks<2, false>)
+                     : (drift ? k_dvr_forward_bricks<4, true> : k_dvr_forward_bricks<4, false>);
+    kern<<<dvr_blocks(B, views, kForwardThreads), kForwardThreads, smem, s>>>(B, K, views, lut, images, trans, work);
+}
+
+// Whether rays of these views drift along an axis (samples_inside): a launch of
+// its own, so that other views do not pay for the look at each run's end
+// (one view of 321x243: 148 -> 150 us).
+static bool views_drift(const mk_dvr_params *views, int nviews) {
+    for (int i = 0; i < nviews; ++i) {
+        const mk_dvr_params &p = views[i];
+        for (int k = 0; k < 3; ++k) {
+            const float d = p.transform[3 * k + 1] * p.scale * p.max_len_spacing[k];
+            if (d != 0.0f && !(fabsf(d * p.step * (float)p.dims[k]) >= 2.0f * kDvrSlow)) return true;
+        }
+    }
+    return false;
 }
 
 // Scratch the caller gave, if it is enough and aligned for these views.
@@ -1320,6 +1348,7 @@ extern "C" int mk_dvr_forward_scratch(const mk_dvr_params *views, int nviews, co
     const size_t npix = (size_t)views[0].width * views[0].height;
     const size_t smem = 2 * (size_t)views[0].lut_len * sizeof(float4);
     const bool bricks = bricks_fit(views, nviews, false, false, scratch, scratch_bytes);
+    const bool drift = bricks && views_drift(views, nviews);
     DvrBricks K = {};
     if (bricks) {
         rc = build_bricks<false>(views[0], volume, lut, scratch, false, K, s);
@@ -1336,7 +1365,7 @@ extern "C" int mk_dvr_forward_scratch(const mk_dvr_params *views, int nviews, co
         dim3 grid((B.W + 31) / 32, (B.H + 7) / 8, count);
         const float4 *l4 = reinterpret_cast<const float4 *>(lut);
         float *im = images + (size_t)first * npix * 3, *tr = transmittance + (size_t)first * npix;
-        if (bricks) launch_forward_bricks(B, K, count, l4, im, tr, workspace, smem, s);
+        if (bricks) launch_forward_bricks(B, K, count, drift, l4, im, tr, workspace, smem, s);
         else k_dvr_forward<<<grid, 256, smem, s>>>(B, volume, l4, im, tr, workspace);
         MK_CUDA_TRY(cudaGetLastError());
     }
@@ -1365,7 +1394,9 @@ extern "C" int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, c
     double *lut_sums = nullptr;
     auto kern = grad_volume ? k_dvr_backward<true, false> : k_dvr_backward<false, false>;
     auto kern_odd = grad_volume ? k_dvr_backward<true, true> : k_dvr_backward<false, true>;
-    auto kern_b = grad_volume ? k_dvr_backward_bricks<true> : k_dvr_backward_bricks<false>;
+    const bool drift = bricks && views_drift(views, nviews);
+    auto kern_b = grad_volume ? (drift ? k_dvr_backward_bricks<true, true> : k_dvr_backward_bricks<true, false>)
+                              : (drift ? k_dvr_backward_bricks<false, true> : k_dvr_backward_bricks<false, false>);
     if (bricks) {
         MK_CUDA_TRY(cudaFuncSetAttribute(kern_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
         MK_CUDA_TRY(cudaFuncSetAttribute(kern_odd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
