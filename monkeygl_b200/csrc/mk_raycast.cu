@@ -77,7 +77,7 @@ constexpr int kRayBlocksPerSm = 6;
 // The hand-off launch: two blocks per SM (up to 128 registers); three and
 // four (80 and 64 registers) were slower on the body frame.
 constexpr int kTailBlocksPerSm = 2;
-template <int MODE, int TRACK, bool COUNT>
+template <int MODE, int TRACK, bool COUNT, bool DRIFT>
 __global__ void __launch_bounds__(256, MODE == kModeVR ? kVrBlocksPerSm : kRayBlocksPerSm)
 k_raycast(RayParams P, cudaTextureObject_t vol, cudaTextureObject_t mask, LabelTable LT, BrickView BV,
           const int *__restrict__ order) {
@@ -95,7 +95,7 @@ k_raycast(RayParams P, cudaTextureObject_t vol, cudaTextureObject_t mask, LabelT
         bx = t % tx;
         by = t / tx;
     }
-    raycast_tile<MODE, TRACK, COUNT>(P, vol, mask, S, BV, s_acc, s_coop, s_px, &s_count, bx, by);
+    raycast_tile<MODE, TRACK, COUNT, DRIFT>(P, vol, mask, S, BV, s_acc, s_coop, s_px, &s_count, bx, by);
     if (MODE == kModeVR && !COUNT && P.tail) {
         __syncthreads();
         if (threadIdx.x == 0) atomicAdd(&P.tail[0], 1u);
@@ -108,7 +108,7 @@ k_raycast(RayParams P, cudaTextureObject_t vol, cudaTextureObject_t mask, LabelT
 // rays into a warp when there are more rays than warps: body 1024^2 frames
 // +1.1%, cardiac +1.9%), writes their pixels, and resets the frame's tail
 // counters for the next frame.
-template <int TRACK>
+template <int TRACK, bool DRIFT>
 __global__ void __launch_bounds__(256, kTailBlocksPerSm) k_vr_tail(RayParams P, cudaTextureObject_t vol, cudaTextureObject_t mask,
                                                  LabelTable LT, BrickView BV) {
     __shared__ LabelSmem S;
@@ -122,7 +122,6 @@ __global__ void __launch_bounds__(256, kTailBlocksPerSm) k_vr_tail(RayParams P, 
     const int tid = threadIdx.x, lane = tid & 31;
     if (P.patch && blockIdx.x == 0 && tid == 0) P.patch[0] = n;
     const unsigned per = 1;    // rays a warp takes at a time
-    const StepVec dv = step_vec(P);
     const float3 L = vr_light(P);
     while (true) {
         unsigned base = 0;
@@ -155,7 +154,7 @@ __global__ void __launch_bounds__(256, kTailBlocksPerSm) k_vr_tail(RayParams P, 
         }
         const unsigned act = __ballot_sync(0xffffffffu, (unsigned)lane < cnt);
         __syncwarp();
-        vr_coop_tail<TRACK, true>(P, vol, mask, S, BV, s_acc, s_coop + (tid & ~31), act, R, dv, L, false);
+        vr_coop_tail<TRACK, DRIFT, true>(P, vol, mask, S, BV, s_acc, s_coop + (tid & ~31), act, R, L, false);
         // the pixel index comes from the spill list: it is checked against
         // the frame before the store, so a corrupt entry cannot write
         // outside the image
@@ -196,7 +195,10 @@ static void launch_mode(const RayParams &P, cudaTextureObject_t vol, cudaTexture
                         const LabelTable &LT, const BrickView &BV, const int *order, cudaStream_t s) {
     const int tx = (P.W + 31) / 32, ty = (P.H + 7) / 8;
     const dim3 grid = order ? dim3(tx * ty) : dim3(tx, ty);
-    k_raycast<MODE, TRACK, COUNT><<<grid, 256, 0, s>>>(P, vol, mask, LT, BV, order);
+    // (only VR frames look at a drift ray by ray)
+    constexpr bool looks = MODE == kModeVR && !COUNT;
+    if (looks && P.drift) k_raycast<MODE, TRACK, COUNT, looks><<<grid, 256, 0, s>>>(P, vol, mask, LT, BV, order);
+    else k_raycast<MODE, TRACK, COUNT, false><<<grid, 256, 0, s>>>(P, vol, mask, LT, BV, order);
 }
 
 template <bool COUNT>
@@ -317,7 +319,7 @@ static int tail_patch(VolumeState &v, RayParams &P, cudaStream_t s, VolumeState:
     return MK_OK;
 }
 
-template <int TRACK>
+template <int TRACK, bool DRIFT>
 static int launch_tail_track(const RayParams &P, cudaTextureObject_t vol, cudaTextureObject_t mask,
                              const LabelTable &LT, const BrickView &BV, cudaStream_t s) {
     // one resident grid; computed once (threads that race here compute the
@@ -328,11 +330,11 @@ static int launch_tail_track(const RayParams &P, cudaTextureObject_t vol, cudaTe
         int dev = 0, sms = 0, per_sm = 0;
         MK_CUDA_TRY(cudaGetDevice(&dev));
         MK_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        MK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vr_tail<TRACK>, 256, 0));
+        MK_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vr_tail<TRACK, DRIFT>, 256, 0));
         grid = std::max(1, sms * std::max(1, per_sm));
         cached.store(grid, std::memory_order_relaxed);
     }
-    k_vr_tail<TRACK><<<grid, 256, 0, s>>>(P, vol, mask, LT, BV);
+    k_vr_tail<TRACK, DRIFT><<<grid, 256, 0, s>>>(P, vol, mask, LT, BV);
     MK_CUDA_TRY(cudaGetLastError());
     return MK_OK;
 }
@@ -340,8 +342,12 @@ static int launch_tail_track(const RayParams &P, cudaTextureObject_t vol, cudaTe
 static int launch_vr_tail(int track, const RayParams &P, cudaTextureObject_t vol, cudaTextureObject_t mask,
                           const LabelTable &LT, const BrickView &BV, cudaStream_t s) {
     if (!P.tail) return MK_OK;
-    if (track == kTrackShared) return launch_tail_track<kTrackShared>(P, vol, mask, LT, BV, s);
-    return launch_tail_track<kTrackNone>(P, vol, mask, LT, BV, s);
+    if (P.drift) {
+        if (track == kTrackShared) return launch_tail_track<kTrackShared, true>(P, vol, mask, LT, BV, s);
+        return launch_tail_track<kTrackNone, true>(P, vol, mask, LT, BV, s);
+    }
+    if (track == kTrackShared) return launch_tail_track<kTrackShared, false>(P, vol, mask, LT, BV, s);
+    return launch_tail_track<kTrackNone, false>(P, vol, mask, LT, BV, s);
 }
 
 std::vector<int> centre_first_tiles(int W, int H, int xT, int yT) {
@@ -519,6 +525,27 @@ int tracking_mode_for(const uint64_t present[2], const float (*params)[3]) {
 
 static int tracking_mode(const VolumeState &v) { return tracking_mode_for(v.present_labels, v.params); }
 
+// Runs of left-out samples (StepVec).  Along an axis that rays only drift along
+// (a camera turned in steps leaves 1e-8 in its matrix) a ray on a brick's face
+// crosses it by one rounding.  With labels the sample beyond has another
+// transfer function and cap, so such an axis ends a run too, unless the ray
+// stays in its layer of bricks (step_vec, in a launch of its own: labelled
+// 512x512x1559 along an axis, 1024^2, 1324 -> 1214 us; the server does without).
+// Without labels the brick's maps hold for half a voxel beyond its faces (the
+// footprint they are made of), and no run drifts as far.
+static void set_brick_steps(RayParams &P, bool labels) {
+    constexpr float kSlowDrift = 1e-4f;     // voxels a coarse step; a run has up to 240
+    P.drift = 0;
+    for (int k = 0; k < 3; ++k) {
+        const float m = (k == 2 && P.invertZ) ? -P.M[7] : P.M[3 * k + 1];
+        const float d = m * P.mls[k] * (P.step1 * P.scale) * P.fdim[k], e = 0.05f;
+        const bool slow = fabsf(d) < kSlowDrift, still = m == 0.0f || (slow && !labels);
+        P.step_rd[k] = still ? 1.0f : 1.0f / copysignf(fmaxf(fabsf(d), 1e-9f), d);
+        P.step_off[k] = still ? kStillAxis : P.step_rd[k] > 0.0f ? kBrick - e : e;
+        if (slow && !still) P.drift |= 1 << k;
+    }
+}
+
 // MIP takes the uniform-window loop when every label present in the mask
 // has alpha > 0 and all of them share one window with ww > 0.
 void set_mip_window(RayParams &P, const uint64_t present[2], const float (*params)[3]) {
@@ -537,6 +564,7 @@ void set_mip_window(RayParams &P, const uint64_t present[2], const float (*param
     P.mip_uniform = 1;
     P.mip_ww = params[first][1];
     P.mip_wl = params[first][2];
+    set_brick_steps(P, false);
 }
 
 int fill_ray_params(const VolumeState &v, const mk_vr_params *p, RayParams &P) {
@@ -602,6 +630,7 @@ int fill_ray_params(const VolumeState &v, const mk_vr_params *p, RayParams &P) {
     P.mip_uniform = 0;
     P.mip_ww = 1.0f;
     P.mip_wl = 0.0f;
+    set_brick_steps(P, v.tex_mask != 0 && p->render_type != MK_RENDER_SURFACE);
     return MK_OK;
 }
 

@@ -71,7 +71,12 @@ struct RayParams {
     int mip_uniform;
     int interior;                // 1: positions are exact enough for the interior of a ray (mip_entries)
     float mip_ww, mip_wl;
+    // the way of the frame's rays through bricks (StepVec), and the axes (bits)
+    // that they drift along (set_brick_steps)
+    float step_rd[3], step_off[3];
+    int drift;
 };
+constexpr float kStillAxis = 1e9f;
 
 struct LabelSmem {
     cudaTextureObject_t tf[MK_MAX_LABELS];
@@ -225,25 +230,38 @@ __device__ __forceinline__ int label_at(cudaTextureObject_t mask, const float3 &
 
 // A ray's way through bricks: coarse steps per voxel along each axis, and the
 // position in a brick (with 0.05 voxels of margin) at which it leaves; an axis
-// it does not move along never ends a run.
+// it does not move along never ends a run (set_brick_steps).
 struct StepVec {
     float3 rd, off;
 };
 
+// For any ray of the frame.
 __device__ __forceinline__ StepVec step_vec(const RayParams &P) {
     StepVec S;
-    const float ds = P.step1 * P.scale, e = 0.05f;
-    const float d[3] = {P.M[1] * P.mls[0] * ds * P.fdim[0], P.M[4] * P.mls[1] * ds * P.fdim[1],
-                        (P.invertZ ? -P.M[7] : P.M[7]) * P.mls[2] * ds * P.fdim[2]};
-    float rd[3], off[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const bool moves = fabsf(d[k]) > 1e-6f;
-        rd[k] = moves ? 1.0f / d[k] : 1.0f;
-        off[k] = !moves ? 1e9f : d[k] > 0.0f ? kBrick - e : e;
+    S.rd = make_float3(P.step_rd[0], P.step_rd[1], P.step_rd[2]);
+    S.off = make_float3(P.step_off[0], P.step_off[1], P.step_off[2]);
+    return S;
+}
+
+__device__ __forceinline__ void still_axis(float p, float q, float &rd, float &off) {
+    if (__fadd_rd(p, kBrickMagic) != __fadd_rd(q, kBrickMagic)) return;
+    rd = 1.0f;
+    off = kStillAxis;
+}
+
+// For one ray's samples from accuLength a0 to a1.  DRIFT: an axis that it drifts
+// along is still where the first and the last lie in the same layer of bricks
+// (all operations of a position are rounded monotonically, so the samples
+// between do as well).
+template <bool DRIFT>
+__device__ __forceinline__ StepVec step_vec(const RayParams &P, float u, float v, float a0, float a1) {
+    StepVec S = step_vec(P);
+    if (DRIFT) {
+        const float3 p = voxel_pos(P, ray_pos(P, u, v, a0)), q = voxel_pos(P, ray_pos(P, u, v, fminf(a1, P.limit)));
+        if (P.drift & 1) still_axis(p.x, q.x, S.rd.x, S.off.x);
+        if (P.drift & 2) still_axis(p.y, q.y, S.rd.y, S.off.y);
+        if (P.drift & 4) still_axis(p.z, q.z, S.rd.z, S.off.z);
     }
-    S.rd = make_float3(rd[0], rd[1], rd[2]);
-    S.off = make_float3(off[0], off[1], off[2]);
     return S;
 }
 
@@ -529,10 +547,10 @@ __device__ __forceinline__ void vr_cap_add(const LabelSmem &S, float (*s_acc)[NT
 // ray's final colour in R.sum.  Groups widen as rays finish: whenever the
 // unfinished rays fit into groups twice as large, their states move to new
 // groups, so a warp's last ray is marched by all 32 lanes.
-template <int TRACK, bool EARLY_TAPS = false, int NT = 256>
+template <int TRACK, bool DRIFT, bool EARLY_TAPS = false, int NT = 256>
 __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTextureObject_t mask,
                              const LabelSmem &S, const BrickView &BV, float (*s_acc)[NT], CoopSample *ws,
-                             unsigned act, VrRay &R, const StepVec &dv, float3 L, bool may_spill) {
+                             unsigned act, VrRay &R, float3 L, bool may_spill) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const float L1 = P.step1, L4 = L1 / 4.0f, L8 = L1 / 8.0f;
@@ -574,6 +592,7 @@ __device__ void vr_coop_tail(const RayParams &P, cudaTextureObject_t vol, cudaTe
             T.done = !member;
             Q = T;
         }
+        const StepVec dv = step_vec<DRIFT>(P, Q.u, Q.v, Q.a - L1, Q.a_stop);
         const int owner_tid = (threadIdx.x & ~31) | owner;
         bool reported = false;
         int round = 0;
@@ -946,7 +965,7 @@ __device__ __forceinline__ float3 vr_light(const RayParams &P) {
 // MonkeyGL's d_render march (core/kernel.cu:156-256) for the ray of this
 // lane, called by every lane of the warp; returns the composited colour
 // (the background where nothing composited).
-template <int TRACK, int NT>
+template <int TRACK, bool DRIFT, int NT>
 __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject_t vol, cudaTextureObject_t mask,
                                            const LabelSmem &S, const BrickView &BV, float (*s_acc)[NT],
                                            CoopSample *ws, bool active, int x, int y) {
@@ -974,7 +993,8 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
             R.done = false;
         }
     }
-    const StepVec dv = step_vec(P);
+    // (refining goes back by less than a coarse step)
+    const StepVec dv = step_vec<DRIFT>(P, R.u, R.v, R.a - P.step1, R.a_stop);
     const float3 L = vr_light(P);
     const float L1 = P.step1;
     const float L4 = L1 / 4.0f;
@@ -1000,7 +1020,7 @@ __device__ __forceinline__ float4 vr_march(const RayParams &P, cudaTextureObject
             if (act == 0u) break;
         }
         if (TRACK != kTrackLocal && __popc(act) <= P.coop_rays) {
-            vr_coop_tail<TRACK>(P, vol, mask, S, BV, s_acc, ws + (tid & ~31), act, R, dv, L, may_spill);
+            vr_coop_tail<TRACK, DRIFT>(P, vol, mask, S, BV, s_acc, ws + (tid & ~31), act, R, L, may_spill);
             break;
         }
         if (!R.done) {
@@ -1139,7 +1159,7 @@ __device__ __forceinline__ int mip_entries(const RayParams &P, cudaTextureObject
 // warp tiles.  s_acc holds the tracked opacity accumulators (kTrackShared),
 // s_px the tile's RGB bytes, s_count the counting-mode total (zeroed by the
 // caller).  Every thread of the block must call it.
-template <int MODE, int TRACK, bool COUNT>
+template <int MODE, int TRACK, bool COUNT, bool DRIFT = false>
 __device__ __forceinline__ void raycast_tile(const RayParams &P, cudaTextureObject_t vol, cudaTextureObject_t mask,
                                              const LabelSmem &S, const BrickView &BV, float (*s_acc)[256],
                                              CoopSample *s_coop, uint8_t (*s_px)[32 * 3],
@@ -1157,7 +1177,7 @@ __device__ __forceinline__ void raycast_tile(const RayParams &P, cudaTextureObje
     float A = 0.0f;   // alphaAcc (VR, MIP max, SURFACE last N.L)
 
     if (MODE == kModeVR && !COUNT) {
-        sum = vr_march<TRACK>(P, vol, mask, S, BV, s_acc, s_coop, active, x, y);
+        sum = vr_march<TRACK, DRIFT>(P, vol, mask, S, BV, s_acc, s_coop, active, x, y);
     } else if (active) {
         const float u = 1.0f * (x - P.W / 2.0f - P.xT) / P.H;
         const float v = 1.0f * (y - P.H / 2.0f - P.yT) / P.H;
