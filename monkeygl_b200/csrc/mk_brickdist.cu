@@ -31,9 +31,9 @@ __device__ __forceinline__ int line_distance(const uint8_t *v, int stride, int i
 }
 
 // x and y of one z slice per block, in shared memory (the maximum distance is
-// separable); latency-bound, a few microseconds.
-__global__ void __launch_bounds__(1024) k_brick_distance_xy(const uint8_t *__restrict__ occupied, int nbx, int nby,
-                                                           uint8_t *__restrict__ out) {
+// separable); latency-bound, a few microseconds.  A block has read its slice
+// before it writes it, so out may be occupied.
+__global__ void __launch_bounds__(1024) k_brick_distance_xy(const uint8_t *occupied, int nbx, int nby, uint8_t *out) {
     extern __shared__ uint8_t smem[];
     const int n = nbx * nby;
     uint8_t *a = smem, *b = smem + n;

@@ -95,6 +95,7 @@ struct VolumeState {
     uint8_t *d_busy = nullptr;               // and the VR busy map
     float *d_mip_tmax = nullptr;
     bool maps_dirty = true;
+    cudaEvent_t maps_ready = nullptr;        // recorded after the maps are built
     uint64_t present_labels[2] = {1, 0};     // labels occurring anywhere in the mask
 
     // ray schedule: accuLength after k plain steps of 1/dim_z
@@ -188,7 +189,12 @@ float float_bound_at(double c);
 // Host helpers shared by the entry points.
 int ensure_device_buffer(VolumeState *v, size_t bytes);
 int ensure_pinned_buffer(VolumeState *v, size_t bytes);
-int rebuild_brick_maps(VolumeState *v, cudaStream_t s);
+// The brick maps of volume v for a launch on stream s: rebuilt there if a table
+// or window changed, after the launches on any stream that read the old ones;
+// else s waits for the stream that built them.
+int ready_brick_maps(VolumeState *v, cudaStream_t s);
+// Make stream s wait for the frames of volume v queued so far on any stream.
+int wait_frames(VolumeState *v, cudaStream_t s);
 // The VR distance map (dist, with scratch tmp) and busy map (busy), a byte per
 // brick each, and the MIP bounds (mip_tmax) of volume v for the given per-label LUT alpha columns
 // (device pointers, nullptr = no table), LUT lengths and (alpha, ww, wl) rows,
@@ -197,7 +203,7 @@ int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha,
                             const float (*params)[3], uint8_t *dist, uint8_t *tmp, uint8_t *busy, float *mip_tmax,
                             cudaStream_t s);
 // Distance map over bricks (mk_brickdist.cu): `occupied` is one byte per brick
-// (0: empty), `tmp` and `dist` one byte per brick each; `dist` may be
+// (0: empty), `tmp` and `dist` one byte per brick each; `tmp` may be
 // `occupied`.  one: no distances, 1 for every empty brick.
 constexpr int kMaxBrickDist = 8;
 int launch_brick_distance(const uint8_t *occupied, int nbx, int nby, int nbz, bool one, uint8_t *tmp, uint8_t *dist,

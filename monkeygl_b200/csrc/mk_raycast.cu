@@ -390,6 +390,20 @@ int wait_table_uses(TableUses &u) {
     return MK_OK;
 }
 
+int wait_frames(VolumeState *v, cudaStream_t s) {
+    // every frame is recorded on the tile order it read
+    for (int i = 0; i < v->n_orders; ++i) {
+        const TableUses &u = v->orders[i].uses;
+        if (u.many) {
+            MK_CUDA_TRY(cudaDeviceSynchronize());
+            for (int k = 0; k < v->n_orders; ++k) free_table_uses(v->orders[k].uses);
+            return MK_OK;
+        }
+        for (int j = 0; j < u.n; ++j) MK_CUDA_TRY(cudaStreamWaitEvent(s, u.done[j], 0));
+    }
+    return MK_OK;
+}
+
 void free_table_uses(TableUses &u) {
     for (int i = 0; i < u.n; ++i) cudaEventDestroy(u.done[i]);
     u.n = 0;
@@ -658,7 +672,7 @@ extern "C" int mk_render_vr(mk_volume vol, const mk_vr_params *params, void *out
         if (rc != MK_OK) return rc;
         P.out = (uint8_t *)v.d_out;
     }
-    rc = rebuild_brick_maps(&v, s);
+    rc = ready_brick_maps(&v, s);
     if (rc != MK_OK) return rc;
     const int *order = nullptr;
     int order_idx = 0, fy_idx = 0;
@@ -755,7 +769,7 @@ extern "C" int mk_count_vr_samples(mk_volume vol, const mk_vr_params *params, ui
     P.skip = 0;
     P.counter = v.d_counter;
     MK_CUDA_TRY(cudaMemsetAsync(v.d_counter, 0, sizeof(unsigned long long), s));
-    rc = rebuild_brick_maps(&v, s);
+    rc = ready_brick_maps(&v, s);
     if (rc != MK_OK) return rc;
     launch_raycast<true>(params->render_type, tracking_mode(v), P, v.tex_linear, v.tex_mask,
                          label_table(&v), brick_view(&v), nullptr, s);
@@ -795,7 +809,7 @@ extern "C" int mk_count_vr_footprint(mk_volume vol, const mk_vr_params *params, 
     P.counter = cnt;
     P.vox_bits = bits;
     P.lab_bits = bits + nwords;
-    rc = rebuild_brick_maps(&v, s);
+    rc = ready_brick_maps(&v, s);
     if (rc == MK_OK) {
         launch_raycast<true>(params->render_type, tracking_mode(v), P, v.tex_linear, v.tex_mask,
                              label_table(&v), brick_view(&v), nullptr, s);

@@ -780,16 +780,26 @@ int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha,
     }
     const int threads = 256;
     const int blocks = (nbricks + threads - 1) / threads;
-    k_brick_visibility<<<blocks, threads, 0, s>>>(v->d_minmax, v->d_labels, nbricks, P, dist, busy, mip_tmax);
+    // (the flags go to the scratch: in the map a byte that is not 0 means empty)
+    k_brick_visibility<<<blocks, threads, 0, s>>>(v->d_minmax, v->d_labels, nbricks, P, dist ? tmp : nullptr, busy,
+                                                  mip_tmax);
     MK_CUDA_TRY(cudaGetLastError());
-    return dist ? launch_brick_distance(dist, v->nb[0], v->nb[1], v->nb[2], one, tmp, dist, s) : MK_OK;
+    return dist ? launch_brick_distance(tmp, v->nb[0], v->nb[1], v->nb[2], one, tmp, dist, s) : MK_OK;
 }
 
-int rebuild_brick_maps(VolumeState *v, cudaStream_t s) {
+int ready_brick_maps(VolumeState *v, cudaStream_t s) {
+    if (!v->maps_ready) MK_CUDA_TRY(cudaEventCreateWithFlags(&v->maps_ready, cudaEventDisableTiming));
+    // (an event never recorded does not hold anything up)
+    MK_CUDA_TRY(cudaStreamWaitEvent(s, v->maps_ready, 0));
     if (!v->maps_dirty) return MK_OK;
-    const int rc = launch_brick_visibility(v, v->d_tf_alpha, v->tf_len, v->params, v->d_dist, v->d_dist_tmp,
-                                           v->d_busy, v->d_mip_tmax, s);
+    int rc = wait_frames(v, s);
+    if (rc == MK_OK)
+        rc = launch_brick_visibility(v, v->d_tf_alpha, v->tf_len, v->params, v->d_dist, v->d_dist_tmp, v->d_busy,
+                                     v->d_mip_tmax, s);
+    // (what a failed build has queued is waited for as well)
+    const cudaError_t e = cudaEventRecord(v->maps_ready, s);
     if (rc != MK_OK) return rc;
+    MK_CUDA_TRY(e);
     v->maps_dirty = false;
     return MK_OK;
 }
@@ -973,7 +983,7 @@ extern "C" int mk_volume_destroy(mk_volume v) {
     cudaFree(st.d_minmax);
     cudaFree(st.d_labels);
     cudaFree(st.d_dist);
-
+    if (st.maps_ready) cudaEventDestroy(st.maps_ready);
     cudaFree(st.d_mip_tmax);
     cudaFree(st.d_accu);
     cudaFree(st.d_out);
