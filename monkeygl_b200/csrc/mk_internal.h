@@ -193,7 +193,8 @@ int ensure_pinned_buffer(VolumeState *v, size_t bytes);
 // or window changed, after the launches on any stream that read the old ones;
 // else s waits for the stream that built them.
 int ready_brick_maps(VolumeState *v, cudaStream_t s);
-// Make stream s wait for the frames of volume v queued so far on any stream.
+// Make stream s wait for the frames of volume v, and the maps they read, queued so
+// far on any stream.
 int wait_frames(VolumeState *v, cudaStream_t s);
 // The VR distance map (dist, with scratch tmp) and busy map (busy), a byte per
 // brick each, and the MIP bounds (mip_tmax) of volume v for the given per-label LUT alpha columns

@@ -391,6 +391,8 @@ int wait_table_uses(TableUses &u) {
 }
 
 int wait_frames(VolumeState *v, cudaStream_t s) {
+    // (an event not recorded yet holds nothing up)
+    if (v->maps_ready) MK_CUDA_TRY(cudaStreamWaitEvent(s, v->maps_ready, 0));
     // every frame is recorded on the tile order it read
     for (int i = 0; i < v->n_orders; ++i) {
         const TableUses &u = v->orders[i].uses;

@@ -788,10 +788,11 @@ int launch_brick_visibility(const VolumeState *v, const float *const *lut_alpha,
 }
 
 int ready_brick_maps(VolumeState *v, cudaStream_t s) {
+    if (!v->maps_dirty) {
+        MK_CUDA_TRY(cudaStreamWaitEvent(s, v->maps_ready, 0));
+        return MK_OK;
+    }
     if (!v->maps_ready) MK_CUDA_TRY(cudaEventCreateWithFlags(&v->maps_ready, cudaEventDisableTiming));
-    // (an event never recorded does not hold anything up)
-    MK_CUDA_TRY(cudaStreamWaitEvent(s, v->maps_ready, 0));
-    if (!v->maps_dirty) return MK_OK;
     int rc = wait_frames(v, s);
     if (rc == MK_OK)
         rc = launch_brick_visibility(v, v->d_tf_alpha, v->tf_len, v->params, v->d_dist, v->d_dist_tmp, v->d_busy,
@@ -1064,6 +1065,9 @@ extern "C" int mk_volume_set_mask(mk_volume v, const uint8_t *labels) {
     const int dx = st.dims[0], dy = st.dims[1], dz = st.dims[2];
     const size_t nvox = (size_t)dx * dy * dz;
     const size_t nbricks = (size_t)st.nb[0] * st.nb[1] * st.nb[2];
+    // frames queued on any stream must have finished reading the old one
+    const int wrc = wait_frames(&st, st.stream);
+    if (wrc != MK_OK) return wrc;
     MK_CUDA_TRY(cudaStreamSynchronize(st.stream));
     free_mask(st);
     st.maps_dirty = true;
@@ -1258,6 +1262,9 @@ extern "C" int mk_volume_set_transfer_function(mk_volume v, int label, const flo
     }
     VolumeState &st = v->st;
     DeviceGuard guard(st.device);
+    // frames queued on any stream must have finished reading the old one
+    const int wrc = wait_frames(&st, st.stream);
+    if (wrc != MK_OK) return wrc;
     MK_CUDA_TRY(cudaStreamSynchronize(st.stream));
     st.maps_dirty = true;
     if (rgba && n_entries > 0 && n_entries == st.tf_len[label] && st.tf_array[label]) {

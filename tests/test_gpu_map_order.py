@@ -85,3 +85,51 @@ def test_a_host_frame_after_a_change(scene):
         assert np.array_equal(vol.render_vr(p[capi.RENDER_VR]), want[capi.RENDER_VR, shown]), f"change {rep}"
     busy.synchronize()
     assert np.array_equal(out.cpu().numpy(), want[capi.RENDER_VR, False])
+
+
+@pytest.mark.parametrize("change", ["table in place", "table of another length", "table removed", "mask", "mask removed"])
+def test_tables_and_masks_change_behind_running_frames(change):
+    """Frames queued on a caller's stream keep the table and the mask they were
+    queued with; the frame after the change has the new one."""
+    ph = make_phantom(DIMS, (0.7, 0.8, 0.9), 5, with_labels=True)
+    c = Camera()
+    c.anterior()
+    c.rotate(25.0, 10.0)
+    p = capi.vr_params(SIZE, SIZE, capi.RENDER_VR, c, DIMS, (0.7, 0.8, 0.9))
+    other = np.where(ph.labels == 0, 1, 0).astype(np.uint8)
+
+    lut = make_tf_lut(TF, 256)
+
+    def base(vol):
+        for l in range(5):
+            vol.set_transfer_function(l, lut * np.float32(0.5 if l == 1 else 1.0))
+        vol.set_mask(ph.labels)
+        vol.set_label_params(_params(True))
+
+    def apply(vol):
+        if change == "table in place":
+            vol.set_transfer_function(0, lut[::-1])
+        elif change == "table of another length":
+            vol.set_transfer_function(0, make_tf_lut(TF, 100)[::-1])
+        elif change == "table removed":
+            vol.set_transfer_function(0, None)
+        else:
+            vol.set_mask(other if change == "mask" else None)
+
+    vol = capi.Volume(ph.volume)
+    base(vol)
+    want = [vol.render_vr(p)]
+    apply(vol)
+    want.append(vol.render_vr(p))
+    assert (want[0] != want[1]).any()
+    base(vol)
+    busy, after = torch.cuda.Stream(), torch.cuda.Stream()
+    frames = [torch.zeros((SIZE, SIZE, 3), dtype=torch.uint8, device="cuda") for _ in range(20)]
+    torch.cuda.synchronize()
+    for f in frames[:-1]:
+        vol.render_vr_device(p, f.data_ptr(), busy.cuda_stream)
+    apply(vol)
+    vol.render_vr_device(p, frames[-1].data_ptr(), after.cuda_stream)
+    torch.cuda.synchronize()
+    for i, f in enumerate(frames):
+        assert np.array_equal(f.cpu().numpy(), want[i == len(frames) - 1]), f"frame {i}"
