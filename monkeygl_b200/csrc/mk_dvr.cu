@@ -865,12 +865,22 @@ __global__ void __launch_bounds__(kForwardThreads) k_dvr_forward_bricks(const __
 
 // The LUT gradient of one ray.  Its colour part is T_i a_i times the pixel's
 // gradient, so a LUT cell needs four sums: (w0, w1) x (T a, dL/da).  They are
-// kept per lane in shared memory for a window of kWin cells about the values
+// kept per lane in shared memory for a window of WIN cells about the values
 // the ray meets (noise about a tissue value stays inside it), so a sample
 // costs one 16-byte read and write without a conflict, and the block's bins
-// are touched only when a ray leaves its window.
-constexpr int kWin = 6;
+// are touched only when a ray leaves its window.  The same noise spans more
+// cells of a longer table: ten from 257 entries on (microseconds a backward with
+// six / ten cells: 256 entries, eight views of 256^2 on 256^3, all visible 3740 /
+// 3897; 500 entries 5503 / 4633, one view of 321x243 1142 / 841, where the plain
+// kernel takes 1091), and six again where the table fills the shared memory (three
+// blocks per SM: 900 entries, 64^3, 1681 / 2050; 256^3 7830 / 8633).
+constexpr int kWinShort = 6, kWinLong = 10;
+constexpr int kWinShortLut = 256, kWinLongLut = 750;
 constexpr int kBackThreads = 128;
+
+static int window_cells(int lut_len) {
+    return lut_len > kWinShortLut && lut_len <= kWinLongLut ? kWinLong : kWinShort;
+}
 
 __device__ __forceinline__ void bin_add(float *bins, int n, int k, float gr, float gg, float gb, const float4 &a) {
     if (a.x != 0.0f) {
@@ -910,7 +920,7 @@ __device__ __forceinline__ void flush_quads(float4 *g, uint32_t cell, const floa
 // views of 256^2; five: 1.52).  The next sample's loads are issued before a
 // sample is summed.  Tried and left: four lanes per ray (2.26 ms; forward 1.14
 // against 0.64: the brick look-ups are then made by every lane).
-template <bool VOLGRAD, bool DRIFT>
+template <bool VOLGRAD, bool DRIFT, int WIN>
 __global__ void __launch_bounds__(kBackThreads, 6)
 k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant__ DvrBricks K, int views,
                       const float4 *__restrict__ lut_g, const float *__restrict__ work,
@@ -919,12 +929,12 @@ k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant_
     extern __shared__ float4 sm[];
     const int n = B.lut_len, tid = threadIdx.x;
     float4 *L = sm, *D = sm + n;
-    float4 *win = sm + 2 * n + tid;      // [kWin][kBackThreads]
-    float *bins = reinterpret_cast<float *>(sm + 2 * n + kWin * kBackThreads);
+    float4 *win = sm + 2 * n + tid;      // [WIN][kBackThreads]
+    float *bins = reinterpret_cast<float *>(sm + 2 * n + WIN * kBackThreads);
     load_lut(lut_g, L, D, n);
     for (int i = tid; i < 4 * n; i += kBackThreads) bins[i] = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kWin; ++k) win[k * kBackThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < WIN; ++k) win[k * kBackThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
 
     const DvrPixel px = dvr_pixel(B, views);
@@ -1019,14 +1029,14 @@ k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant_
         U = q.w * p + d * U;
         // LUT sums
         int slot = h.k - wbase;
-        if ((unsigned)slot >= (unsigned)kWin) {
+        if ((unsigned)slot >= (unsigned)WIN) {
             while (used) {
                 const int u = __ffs(used) - 1;
                 used &= used - 1u;
                 bin_add(bins, n, wbase + u, gr, gg, gb, win[u * kBackThreads]);
                 win[u * kBackThreads] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            wbase = max(h.k - kWin / 2, 0);
+            wbase = max(h.k - WIN / 2, 0);
             slot = h.k - wbase;
         }
         used |= 1u << slot;
@@ -1077,7 +1087,7 @@ k_dvr_backward_bricks(const __grid_constant__ DvrBatch B, const __grid_constant_
     if (VOLGRAD) flush_quads(K.gquads, cell, va);
     __syncwarp();
 #pragma unroll 1
-    for (int u = 0; u < kWin; ++u) {
+    for (int u = 0; u < WIN; ++u) {
         const bool has = (used >> u) & 1u;
         const float4 a = win[u * kBackThreads];
         const float4 a0 = make_float4(gr * a.x, gg * a.x, gb * a.x, a.z), a1 = make_float4(gr * a.y, gg * a.y, gb * a.y, a.w);
@@ -1202,7 +1212,11 @@ static BrickLayout brick_layout(const int dims[3], bool gradients) {
 // 640 / 460 us; eight 128^2 views of 64^3, six million samples: 644 / 473 us),
 // and for the backward the LUT must have 64 entries: with a few, long runs in
 // one LUT cell make the plain one cheap (16 entries, 249x73x51, rays of 250:
-// 215 / 316 us a step).  The exit model
+// 215 / 316 us a step).  With a long table few blocks fit an SM: above 750
+// entries the backward needs four samples per voxel (800 entries, one view of
+// 321x243 on 211x190x157, two per voxel: 1298 / 1443 us; 128^3, six: 1612 / 1304),
+// and without voxel gradients, whose reductions make the plain kernel dear, above
+// 512 long rays (600 entries, 64^3, rays of 107: 1323 / 1479 us).  The exit model
 // of a ray (linear in the sample number) holds to a few hundredths of a cell
 // while a unit of the ray parameter is at most 3e4 cells along an axis; quads
 // are addressed with 32 bits.
@@ -1210,9 +1224,11 @@ constexpr double kDvrSamplesPerVoxel = 0.25;
 constexpr double kDvrManySamples = 5.0e6;
 constexpr double kDvrLongRay = 240.0;
 constexpr int kDvrLongLut = 64;
+constexpr int kDvrLutOnlyLut = 512;
+constexpr double kDvrLongLutSamplesPerVoxel = 4.0;
 constexpr double kDvrMaxCellsPerUnit = 3.0e4;
 
-static bool use_bricks(const mk_dvr_params *views, int nviews, bool backward) {
+static bool use_bricks(const mk_dvr_params *views, int nviews, bool backward, bool gradients) {
     const mk_dvr_params &a = views[0];
     double samples = 0.0, depth = 0.0;
     for (int i = 0; i < nviews; ++i) {
@@ -1239,7 +1255,9 @@ static bool use_bricks(const mk_dvr_params *views, int nviews, bool backward) {
     const BrickLayout l = brick_layout(a.dims, false);
     if (l.nb[1] > 65535 || l.nb[2] > 65535 || l.n * kDvrBrickQuads >= 0xffffffffull) return false;
     if (samples < kDvrManySamples && (depth < kDvrLongRay || (backward && a.lut_len < kDvrLongLut))) return false;
-    return samples >= kDvrSamplesPerVoxel * a.dims[0] * a.dims[1] * (double)a.dims[2];
+    if (backward && !gradients && a.lut_len > kDvrLutOnlyLut && depth < kDvrLongRay) return false;
+    const double per_voxel = backward && a.lut_len > kWinLongLut ? kDvrLongLutSamplesPerVoxel : kDvrSamplesPerVoxel;
+    return samples >= per_voxel * a.dims[0] * a.dims[1] * (double)a.dims[2];
 }
 
 // Build the bricks of `volume` under `lut` in `scratch`, and their distances.
@@ -1271,11 +1289,14 @@ static unsigned dvr_blocks(const DvrBatch &B, int views, int threads) {
     return ((B.W + 15) / 16) * ((B.H + h - 1) / h) * (unsigned)views;
 }
 
-// Samples whose loads a ray has in flight: four where the launch is too small
-// to fill the SMs and the longest rays set its time (one view of 321x243:
-// 107 us, against 118 with two and 150 with one), two where there are rays
-// enough (eight views of 256^2: 638 us, against 670 with four, whose registers
-// cost resident warps, and 686 with one).  The line: about 2000 rays per SM.
+// Samples whose loads a ray has in flight: four where the launch is too small to
+// fill the SMs and the longest rays set its time, two where there are rays enough
+// (four cost registers, and so resident warps).  One to 32 views of 128^2 to 700^2
+// on three volumes, mostly transparent and all visible: up to 130,000 rays four
+// take 1-18% less (one view of 321x243: 107 us, against 118 with two and 150 with
+// one), from 150,000 on the two are level within 5%, either way by volume and
+// table, with two ahead by more in the largest launches (eight views of 256^2 on
+// 256^3: 638 us, against 670 and 686 with one).  The line is in that level stretch.
 constexpr long long kDvrManyRays = 300000;
 
 static void launch_forward_bricks(const DvrBatch &B, const DvrBricks &K, int views, bool drift, const float4 *lut,
@@ -1284,6 +1305,15 @@ static void launch_forward_bricks(const DvrBatch &B, const DvrBricks &K, int vie
     auto kern = many ? (drift ? k_dvr_forward_bricks<2, true> : k_dvr_forward_bricks<2, false>)
                      : (drift ? k_dvr_forward_bricks<4, true> : k_dvr_forward_bricks<4, false>);
     kern<<<dvr_blocks(B, views, kForwardThreads), kForwardThreads, smem, s>>>(B, K, views, lut, images, trans, work);
+}
+
+static decltype(&k_dvr_backward_bricks<true, true, kWinLong>) backward_bricks(bool volgrad, bool drift, bool wide) {
+    if (volgrad) {
+        if (drift) return wide ? k_dvr_backward_bricks<true, true, kWinLong> : k_dvr_backward_bricks<true, true, kWinShort>;
+        return wide ? k_dvr_backward_bricks<true, false, kWinLong> : k_dvr_backward_bricks<true, false, kWinShort>;
+    }
+    if (drift) return wide ? k_dvr_backward_bricks<false, true, kWinLong> : k_dvr_backward_bricks<false, true, kWinShort>;
+    return wide ? k_dvr_backward_bricks<false, false, kWinLong> : k_dvr_backward_bricks<false, false, kWinShort>;
 }
 
 // Whether rays of these views drift along an axis (samples_inside): a launch of
@@ -1303,7 +1333,7 @@ static bool views_drift(const mk_dvr_params *views, int nviews) {
 // Scratch the caller gave, if it is enough and aligned for these views.
 static bool bricks_fit(const mk_dvr_params *views, int nviews, bool backward, bool gradients, const void *scratch,
                        size_t bytes) {
-    return scratch && (reinterpret_cast<uintptr_t>(scratch) & 255) == 0 && use_bricks(views, nviews, backward) &&
+    return scratch && (reinterpret_cast<uintptr_t>(scratch) & 255) == 0 && use_bricks(views, nviews, backward, gradients) &&
            bytes >= brick_layout(views[0].dims, gradients).bytes;
 }
 
@@ -1331,7 +1361,7 @@ extern "C" int mk_dvr_scratch_bytes(const mk_dvr_params *views, int nviews, int 
     }
     int rc = check_views(views, nviews);
     if (rc != MK_OK) return rc;
-    *bytes = use_bricks(views, nviews, gradients != 0) ? brick_layout(views[0].dims, gradients != 0).bytes : 0;
+    *bytes = use_bricks(views, nviews, gradients != 0, gradients != 0) ? brick_layout(views[0].dims, gradients != 0).bytes : 0;
     return MK_OK;
 }
 
@@ -1389,14 +1419,14 @@ extern "C" int mk_dvr_backward_scratch(const mk_dvr_params *views, int nviews, c
     cudaStream_t s = (cudaStream_t)stream;
     const size_t npix = (size_t)views[0].width * views[0].height;
     const bool bricks = bricks_fit(views, nviews, true, grad_volume != nullptr, scratch, scratch_bytes);
-    const size_t smem = 3 * (size_t)views[0].lut_len * sizeof(float4), smem_b = smem + kWin * kBackThreads * sizeof(float4);
+    const int win = window_cells(views[0].lut_len);
+    const size_t smem = 3 * (size_t)views[0].lut_len * sizeof(float4), smem_b = smem + win * kBackThreads * sizeof(float4);
     DvrBricks K = {};
     double *lut_sums = nullptr;
     auto kern = grad_volume ? k_dvr_backward<true, false> : k_dvr_backward<false, false>;
     auto kern_odd = grad_volume ? k_dvr_backward<true, true> : k_dvr_backward<false, true>;
     const bool drift = bricks && views_drift(views, nviews);
-    auto kern_b = grad_volume ? (drift ? k_dvr_backward_bricks<true, true> : k_dvr_backward_bricks<true, false>)
-                              : (drift ? k_dvr_backward_bricks<false, true> : k_dvr_backward_bricks<false, false>);
+    auto kern_b = backward_bricks(grad_volume != nullptr, drift, win == kWinLong);
     if (bricks) {
         MK_CUDA_TRY(cudaFuncSetAttribute(kern_b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b));
         MK_CUDA_TRY(cudaFuncSetAttribute(kern_odd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
