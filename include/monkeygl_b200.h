@@ -332,8 +332,10 @@ int mk_dvr_backward(const mk_dvr_params *views, int nviews, const float *volume,
  * several times faster for all but small images of large volumes.  Results
  * are those of the plain calls (images and workspace bit for bit; gradients
  * up to the order of their sums).  mk_dvr_scratch_bytes gives the bytes, 0
- * where the plain calls are as fast; gradients = 1 for a backward call with
- * grad_volume.  With less (or NULL) scratch they are the plain calls. */
+ * where the plain calls are as fast; gradients = 0 for a forward call, 1 for a
+ * backward call with grad_volume, 2 for one without.  It is 9216 bytes per 8^3
+ * voxels (18 a voxel: 0.33 GB for 256^3), twice that with grad_volume.  With
+ * less (or NULL) scratch they are the plain calls. */
 int mk_dvr_scratch_bytes(const mk_dvr_params *views, int nviews, int gradients, size_t *bytes);
 int mk_dvr_forward_scratch(const mk_dvr_params *views, int nviews, const float *volume, const float *lut,
                            float *images, float *transmittance, float *workspace, void *scratch,

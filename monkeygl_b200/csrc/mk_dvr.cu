@@ -1361,7 +1361,8 @@ extern "C" int mk_dvr_scratch_bytes(const mk_dvr_params *views, int nviews, int 
     }
     int rc = check_views(views, nviews);
     if (rc != MK_OK) return rc;
-    *bytes = use_bricks(views, nviews, gradients != 0, gradients != 0) ? brick_layout(views[0].dims, gradients != 0).bytes : 0;
+    const bool backward = gradients != 0, volgrad = backward && gradients != 2;
+    *bytes = use_bricks(views, nviews, backward, volgrad) ? brick_layout(views[0].dims, volgrad).bytes : 0;
     return MK_OK;
 }
 

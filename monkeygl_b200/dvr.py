@@ -76,20 +76,34 @@ def workspace_floats(views) -> int:
     return out.value
 
 
+# The pass that scratch is for (mk_dvr_scratch_bytes).
+_FORWARD, _BACKWARD, _BACKWARD_LUT = 0, 1, 2
+_LARGE_SCRATCH = 2 << 30
+
+
+def _scratch(arr, nv, what, device):
+    """Scratch for one call on the current stream (which the caching allocator
+    hands the memory back to), or none.  It takes 18 or 36 bytes a voxel, so a large
+    one is only asked for if it leaves half of the memory there is to have: the
+    program around keeps room, and an allocation that would fail does not make
+    torch empty its cache on every call."""
+    import torch
+    n = C.c_size_t(0)
+    _check(_lib().mk_dvr_scratch_bytes(arr, nv, what, C.byref(n)), "mk_dvr_scratch_bytes")
+    if n.value == 0:
+        return None, 0
+    if n.value >= _LARGE_SCRATCH and not torch.cuda.is_current_stream_capturing():
+        room = torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+        if n.value > room // 2:
+            return None, 0
+    try:
+        return torch.empty(n.value, dtype=torch.uint8, device=device), n.value
+    except torch.cuda.OutOfMemoryError:
+        return None, 0
+
+
 def _torch_function():
     import torch
-
-    def scratch(arr, nv, gradients, device):
-        """Scratch for one call on the current stream (which the caching
-        allocator hands the memory back to), or none if it does not fit."""
-        n = C.c_size_t(0)
-        _check(_lib().mk_dvr_scratch_bytes(arr, nv, int(gradients), C.byref(n)), "mk_dvr_scratch_bytes")
-        if n.value == 0:
-            return None, 0
-        try:
-            return torch.empty(n.value, dtype=torch.uint8, device=device), n.value
-        except torch.cuda.OutOfMemoryError:
-            return None, 0
 
     class VolumeRender(torch.autograd.Function):
         @staticmethod
@@ -117,7 +131,7 @@ def _torch_function():
             work = None
             if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
                 work = torch.empty(workspace_floats(arr), dtype=torch.float32, device=volume.device)
-            tmp, tmp_bytes = scratch(arr, nv, False, volume.device)
+            tmp, tmp_bytes = _scratch(arr, nv, _FORWARD, volume.device)
             _check(L.mk_dvr_forward_scratch(arr, nv, _ptr(volume), _ptr(lut), _ptr(images), _ptr(trans), _ptr(work),
                                             _ptr(tmp), tmp_bytes, stream), "mk_dvr_forward")
             ctx.views = arr
@@ -133,7 +147,8 @@ def _torch_function():
             grad_lut = torch.zeros_like(lut)
             grad_vol = torch.zeros_like(volume) if ctx.needs_input_grad[0] else None
             g = grad_images.contiguous().float()
-            tmp, tmp_bytes = scratch(ctx.views, len(ctx.views), grad_vol is not None, volume.device)
+            what = _BACKWARD_LUT if grad_vol is None else _BACKWARD
+            tmp, tmp_bytes = _scratch(ctx.views, len(ctx.views), what, volume.device)
             _check(L.mk_dvr_backward_scratch(ctx.views, len(ctx.views), _ptr(volume), _ptr(lut), _ptr(ctx.work), _ptr(g),
                                              _ptr(grad_lut), _ptr(grad_vol), _ptr(tmp), tmp_bytes, stream),
                    "mk_dvr_backward")
