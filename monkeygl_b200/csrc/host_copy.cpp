@@ -5,11 +5,16 @@
 // memory latency (measured 24 us for 512 KB, 47 us for 1 MB, 200 us for 3 MB,
 // against 10 / 19 / 55 us for the DMA itself).  Up to three helper threads,
 // kept by the process and asleep between images, are woken while the GPU still
-// works and then share the copy in 64 KB pieces with the calling thread.  The
-// caller takes pieces too and needs no helper to finish: one that wakes late,
-// or no longer exists (a forked child), finds or leaves nothing to do.  One
-// caller at a time has the helpers; another copies alone.
+// works and then share the copy in 64 KB pieces with the calling thread.  They
+// look for it for 200 us and go back to sleep: an image that comes later than
+// that is copied by the caller alone.  The caller takes pieces until none is
+// left, so a helper that wakes late leaves nothing undone; it waits only for
+// pieces that a helper is copying, and gives up its core meanwhile if that takes
+// long (the helper may want it).  One caller at a time has the helpers; another
+// copies alone, and so does a forked child, which has no helpers and whose
+// copies of the locks may be held for good.
 #include <string.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -29,7 +34,7 @@ namespace {
 constexpr size_t kPiece = 64u << 10;
 constexpr size_t kHelpMin = 256u << 10;     // smaller images: the caller alone
 constexpr int kHelpers = 3;
-constexpr auto kSpin = std::chrono::microseconds(200);
+constexpr auto kSpin = std::chrono::microseconds(200), kWait = std::chrono::microseconds(50);
 
 inline void pause_cpu() {
 #if defined(__x86_64__)
@@ -40,6 +45,7 @@ inline void pause_cpu() {
 }
 
 struct CopyPool {
+    const pid_t process = getpid();
     std::mutex owner;                        // held by the caller that has the helpers
     std::mutex mu;
     std::condition_variable cv;
@@ -99,9 +105,18 @@ struct CopyPool {
     }
 };
 
+// The process's pool; null in a forked child, and for a caller that comes while
+// another makes it.  No lock: one held at a fork would be held in the child.
 CopyPool *pool() {
-    static CopyPool *p = new (std::nothrow) CopyPool();   // kept until the process exits, like its threads
-    return p;
+    static std::atomic<CopyPool *> made{nullptr};     // kept until the process exits, like its threads
+    static std::atomic<bool> making{false};
+    CopyPool *p = made.load(std::memory_order_acquire);
+    if (!p) {
+        if (making.exchange(true, std::memory_order_acq_rel)) return nullptr;
+        p = new (std::nothrow) CopyPool();
+        made.store(p, std::memory_order_release);
+    }
+    return p && p->process == getpid() ? p : nullptr;
 }
 
 }  // namespace
@@ -132,7 +147,13 @@ void copy_out(void *dst, const void *src, size_t bytes) {
     p->ticket.store((uint64_t)gen << 32 | n, std::memory_order_release);
     while (p->take(gen)) {
     }
-    while (p->done.load(std::memory_order_acquire) != n) pause_cpu();
+    const auto until = std::chrono::steady_clock::now() + kWait;
+    bool yield = false;
+    for (int i = 1; p->done.load(std::memory_order_acquire) != n; ++i) {
+        if (yield) std::this_thread::yield();
+        else pause_cpu();
+        if (!yield && (i & 63) == 0) yield = std::chrono::steady_clock::now() > until;
+    }
     p->owner.unlock();
 }
 
