@@ -45,3 +45,18 @@ def test_cameras_turned_in_steps_match_plain(n, turns, by):
     for k in range(3):
         assert torch.equal(a[k], b[k]), ("image", "transmittance", "workspace")[k]
     assert _close(b[3], a[3]) and _close(b[4], a[4])
+
+
+@pytest.mark.parametrize("by", [(90.0001, 0.0), (90.003, 0.0), (179.994, 0.0), (0.0, 89.9995), (90.02, 0.0), (90.06, 0.0)])
+@pytest.mark.parametrize("n,air", [(128, False), (121, True)])
+def test_cameras_close_to_an_axis_match_plain(n, air, by):
+    """Drifts of 1e-6 to 5e-4 cells a sample, on both sides of the rate below which
+    the end of a run is looked at."""
+    dims, lut = (n, n, n), 64
+    views = [dvr.dvr_params(2 * n, 2 * n, _turned(1, by), dims, (1.0, 1.0, 1.0), 0.5, 0.0, lut)]
+    vol, table = _volume(dims, 3, air=air), _lut(lut, "cut", 4)
+    g = torch.randn((1, 2 * n, 2 * n, 3), generator=torch.Generator("cuda").manual_seed(5), device="cuda")
+    a, b = (_run(views, vol, table, g, bricks, True) for bricks in (False, True))
+    for k in range(3):
+        assert torch.equal(a[k], b[k]), ("image", "transmittance", "workspace")[k]
+    assert _close(b[3], a[3]) and _close(b[4], a[4])

@@ -82,3 +82,32 @@ def test_cameras_turned_in_steps_mip_and_surface(kind, turns, by, axis):
     images = [vol.render_vr(capi.vr_params(2 * N, 2 * N, kind, c, (N, N, N), (1.0, 1.0, 1.0), flags=f))
               for f in (0, capi.VR_NO_SKIP)]
     assert np.array_equal(images[0], images[1])
+
+
+@pytest.mark.parametrize("labelled", [False, True])
+@pytest.mark.parametrize("kind", [capi.RENDER_VR, capi.RENDER_MIP, capi.RENDER_SURFACE])
+@pytest.mark.parametrize("by", [(90.0001, 0.0), (90.003, 0.0), (179.994, 0.0), (0.0, 89.9995), (90.02, 0.0)])
+def test_cameras_close_to_an_axis(labelled, kind, by):
+    """Drifts of 2e-6 to 3e-4 voxels a step, on both sides of the rate below which
+    an axis is looked at ray by ray (or, without labels, counts as still)."""
+    rng = np.random.default_rng(12)
+    v = np.full((N, N, N), -900, np.int16)
+    v[40:88, 30:100, 24:104] = rng.integers(-300, 1400, (48, 70, 80))
+    vol = capi.Volume(v)
+    lp = np.zeros((capi.MAX_LABELS, 3), np.float32)
+    lp[:, 1] = 1.0
+    lp[:3] = (1.0, 1700.0, 650.0)
+    if labelled:
+        vol.set_mask(_labels(1, False))
+        lp[1] = (0.3, 1700.0, 650.0)
+    for l in range(3):
+        vol.set_transfer_function(l, make_tf_lut(FAINT if l == 2 else PLAIN, 256) *
+                                  (np.arange(256) > 90)[:, None].astype(np.float32))
+    vol.set_label_params(lp)
+    c = Camera()
+    c.anterior()
+    c.rotate(*by)
+    images = [vol.render_vr(capi.vr_params(2 * N, 2 * N, kind, c, (N, N, N), (1.0, 1.0, 1.0), flags=f))
+              for f in (0, capi.VR_NO_SKIP)]
+    assert (images[1] != images[1][0, 0]).any()
+    assert np.array_equal(images[0], images[1]), f"{np.count_nonzero(images[0] != images[1])} bytes differ"
