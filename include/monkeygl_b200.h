@@ -146,7 +146,9 @@ const char *mk_version(void);
  * may be freed after the call returns.  A volume handle is used from one host
  * thread at a time (its per-frame caches -- tile orders, ray parameter
  * tables, hand-off lists -- are not locked); concurrent renders of one volume
- * go through several streams from that thread, or through mk_server_*.
+ * go through several streams from that thread, or through mk_server_*.  Tables,
+ * masks and label parameters may change between them: a frame has those that
+ * were set when it was queued, whatever stream it is on.
  * The brick maps are built by kernels whose waits are bounded: a wait that
  * runs out (never expected) is reported as MK_ERR_TIMEOUT and no volume is
  * returned.

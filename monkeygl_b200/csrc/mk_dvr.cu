@@ -486,8 +486,8 @@ __global__ void __launch_bounds__(128) k_dvr_backward(const __grid_constant__ Dv
 // the kernels above run at the rate at which the load/store unit takes lines
 // (about 190 cycles per warp and sample, 99% of L1TEX).  On 256^3 with eight
 // views of 256^2 the rearrangement takes 66-77 us, the forward 640 us (plain:
-// 5.2 ms) and the backward 1430 us (plain: 6.2 ms); the load/store unit (78%)
-// and instruction issue (73%) now share the bound.  Here a cell's plane
+// 5.2 ms) and the backward 1430 us (plain: 6.2 ms); the load/store unit (93%)
+// and instruction issue (78%) now share the forward's bound.  Here a cell's plane
 // of four voxels is one float4 ("quad"), so a sample is two 16-byte loads;
 // a 128-byte line holds 4x2 cells of one plane, and a quarter warp (the lanes
 // a 16-byte load serves together) covers 4x2 pixels.
